@@ -19,10 +19,12 @@
 // The grid barriers are this file's own (not cooperative_groups::grid_group::
 // sync) so that their waits are bounded: if the other blocks never arrive
 // they record an error in DevScalars::error and every block leaves the
-// solver.  The context's solvers count arrivals on a counter that the host
-// zeroes before each launch (grid_barrier_counted: a fence, one atomic and
-// the poll that sees the total); the no-allocation entry point's pressure
-// solve keeps the generation barrier (grid_barrier), which needs no reset.
+// solver.  Ranges larger than one cell per resident thread count arrivals on
+// a counter that the host zeroes before each launch (grid_barrier_counted: a
+// fence, one atomic and the poll that sees the total).  Ranges of at most one
+// cell per resident thread keep the whole solve in registers and exchange
+// their sums through slots that are barrier and reduction in one
+// (grid_exchange).
 #include "pvof_device.cuh"
 #include "pvof_kernels.cuh"
 
@@ -30,54 +32,14 @@ namespace pvof {
 
 constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;
 
-struct GridSync {
-    DevScalars *s;
-    unsigned nblocks;
-};
-
-// Returns false (in every thread of the block) when the barrier gave up.
-__device__ __noinline__ bool grid_barrier(const GridSync &gs)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *vgen = &gs.s->bar_gen;
-        volatile int *verr = &gs.s->error;
-        int good = (*verr == 0);
-        unsigned g = *vgen;
-        __threadfence();
-        unsigned arrived = atomicAdd(&gs.s->bar_count, 1u);
-        if (arrived == gs.nblocks - 1) {
-            gs.s->bar_count = 0u;
-            __threadfence();
-            atomicAdd(&gs.s->bar_gen, 1u);
-        } else {
-            unsigned long long spins = 0;
-            while (*vgen == g) {
-                ++spins;
-                if ((spins & 1023ull) == 0 && (*verr != 0 || spins > BARRIER_SPIN_LIMIT)) {
-                    atomicCAS(&gs.s->error, 0, 1);   // 1: a grid-wide solver's barrier
-                    good = 0;
-                    break;
-                }
-                if (spins > 4096) __nanosleep(64);
-            }
-        }
-        __threadfence();
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 // Grid barrier on a counter of arrivals that the host zeroes before the
 // launch: the g-th barrier of a launch is passed once the counter reaches
 // g * gridDim.x.  Each block's thread 0 publishes the block's writes
 // (block barrier, then a device-scope fence), adds its arrival without
 // waiting for the result and polls the counter; nothing is reset or bumped
 // after the last arrival, so the barrier costs a fence, one atomic and the
-// poll that sees the total.  Bounded like grid_barrier: false (in every
-// thread of the block) when it gave up, with the error recorded.
+// poll that sees the total.  Bounded: false (in every thread of the block)
+// when it gave up, with the error recorded.
 __device__ __noinline__ bool grid_barrier_counted(unsigned long long *arrivals, int *error, unsigned long long target)
 {
     __shared__ int ok;
@@ -158,6 +120,140 @@ __device__ __forceinline__ void put_partial(double *part, double v)
 {
     double s = block_sum(v);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
+}
+
+// Grid-wide sum and barrier in one: every block publishes its partial sums in
+// a slot of its own, tagged with the number of the exchange (the epoch).  On
+// at most 32 blocks every block polls all slots until they carry that tag; on
+// more, block 0 does and publishes the totals in one more slot, which the
+// other blocks poll (all blocks polling all slots crowds the few L2 lines the
+// slots lie in).  One or two one-way trips through L2 replace
+// grid_barrier_counted's atomic, its poll and the load of the partials behind
+// it.  Measured, B200, us per exchange without and with PUBLISH: 9 blocks
+// of 512 threads 0.97 and 1.9, counted barrier and partials 2.5; 227 blocks
+// 2.1 and 3.2, every block polling 4.4 and 5.3, counted 6.3.
+// A slot holds each double as two words of 32 value bits and the 32-bit
+// epoch, so a word is valid by itself and the two need not arrive together.
+// Two buffers alternate: a block writes epoch e + 2 only after it has the
+// totals of e + 1, which need every block's e + 1, published after it read e.
+// The host zeroes the slots before each launch; epochs start at 1.  The sums
+// are taken in put_partial's and grid_total's order, so the totals are theirs
+// bit for bit.
+// PUBLISH: the block's earlier stores to global memory are visible to every
+// block after the exchange (else only the sums are exchanged): a fence before
+// the block's slot is written, acquiring loads once a slot has been seen, and
+// a fence in block 0 before the totals.  False, in every thread of the block,
+// when the bounded wait gave up.
+struct Slots {
+    unsigned long long *w;   // two buffers of gridDim.x + 1 slots
+    int *error;
+    unsigned epoch;
+};
+
+constexpr unsigned ALL_POLL_BLOCKS = 32;
+constexpr int SLOT_BLOCKS = 512;   // most blocks: one slot per thread of block 0
+
+__device__ __forceinline__ void slot_put(unsigned long long *p, double v, unsigned e)
+{
+    const unsigned long long x = (unsigned long long)__double_as_longlong(v), tag = (unsigned long long)e << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((x & 0xffffffffull) | tag), "l"((x >> 32) | tag)
+                 : "memory");
+}
+
+// waits (bounded) for epoch e in slot p
+template <bool ACQUIRE>
+__device__ __forceinline__ bool slot_get(const unsigned long long *p, unsigned e, double &v, int *error)
+{
+    unsigned long long lo, hi, spins = 0;
+    for (;;) {
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+        if ((unsigned)(lo >> 32) == e && (unsigned)(hi >> 32) == e) break;
+        ++spins;
+        if ((spins & 1023ull) == 0 && (*(volatile int *)error != 0 || spins > BARRIER_SPIN_LIMIT)) {
+            atomicCAS(error, 0, 1);   // 1: a grid-wide solver's barrier
+            return false;
+        }
+        if (spins > 4096) __nanosleep(64);
+    }
+    if (ACQUIRE) {
+        unsigned long long seen;
+        asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(seen) : "l"(p) : "memory");
+    }
+    v = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
+    return true;
+}
+
+template <int NV, bool PUBLISH>
+__device__ __forceinline__ bool grid_exchange(Slots &sl, double (&v)[NV])
+{
+    __shared__ double wsum[32][NV], vals[NV][SLOT_BLOCKS], total[NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned nb = gridDim.x, e = ++sl.epoch;
+    unsigned long long *buf = sl.w + (size_t)(e & 1u) * (nb + 1) * 2 * NV;
+    int good = 1;
+#pragma unroll
+    for (int n = 0; n < NV; n++)
+        for (int o = 16; o > 0; o >>= 1) v[n] += __shfl_down_sync(0xffffffffu, v[n], o);
+    if (lane == 0)
+#pragma unroll
+        for (int n = 0; n < NV; n++) wsum[warp][n] = v[n];
+    __syncthreads();
+    if (warp == 0) {
+        double b[NV];
+#pragma unroll
+        for (int n = 0; n < NV; n++) {
+            b[n] = lane < (int)(blockDim.x >> 5) ? wsum[lane][n] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) b[n] += __shfl_down_sync(0xffffffffu, b[n], o);
+        }
+        if (lane == 0) {
+            if (PUBLISH) __threadfence();
+#pragma unroll
+            for (int n = 0; n < NV; n++) slot_put(buf + ((size_t)blockIdx.x * NV + n) * 2, b[n], e);
+        }
+        __syncwarp();
+    }
+    if (nb <= ALL_POLL_BLOCKS) {
+        if (warp == 0) {
+#pragma unroll
+            for (int n = 0; n < NV; n++) {
+                double t = 0.0;
+                if (lane < (int)nb && !slot_get<PUBLISH>(buf + ((size_t)lane * NV + n) * 2, e, t, sl.error)) good = 0;
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) total[n] = t;
+            }
+        }
+    } else if (blockIdx.x == 0) {
+        for (unsigned q = threadIdx.x; q < nb; q += blockDim.x)
+#pragma unroll
+            for (int n = 0; n < NV; n++)
+                if (!slot_get<PUBLISH>(buf + ((size_t)q * NV + n) * 2, e, vals[n][q], sl.error)) good = 0;
+        __syncthreads();
+        if (warp == 0) {
+            double t[NV];
+#pragma unroll
+            for (int n = 0; n < NV; n++) {
+                t[n] = 0.0;
+                for (unsigned q = lane; q < nb; q += 32) t[n] += vals[n][q];
+                for (int o = 16; o > 0; o >>= 1) t[n] += __shfl_xor_sync(0xffffffffu, t[n], o);
+            }
+            if (lane == 0) {
+                if (PUBLISH) __threadfence();
+#pragma unroll
+                for (int n = 0; n < NV; n++) {
+                    slot_put(buf + ((size_t)nb * NV + n) * 2, t[n], e);
+                    total[n] = t[n];
+                }
+            }
+        }
+    } else if (threadIdx.x == 0) {
+#pragma unroll
+        for (int n = 0; n < NV; n++)
+            if (!slot_get<PUBLISH>(buf + ((size_t)nb * NV + n) * 2, e, total[n], sl.error)) good = 0;
+    }
+    good = __syncthreads_and(good);
+#pragma unroll
+    for (int n = 0; n < NV; n++) v[n] = total[n];
+    return good != 0;
 }
 
 struct Range {
@@ -295,6 +391,122 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
 }
 
 // ---------------------------------------------------------------------------
+// One cell per thread: every value of the solve that belongs to the cell stays
+// in the thread's registers, the direction at the four stencil neighbours
+// included (each thread advances d = z + beta d at all five points, the same
+// operation on the same operands as the owner's), so an iteration moves one
+// store of z and four loads of the neighbours' z per cell through L2 and is
+// bound by the latency of its two grid-wide sums.  The sum behind the step
+// length needs no data of other blocks and skips the fences.  Iterates and
+// sums are those of the grid-stride passes, bit for bit.
+// ---------------------------------------------------------------------------
+
+// the velocity solve with one cell per thread (B200, 241x482: 13.9 -> 9.2 us
+// per iteration)
+__global__ void __launch_bounds__(512, 2) k_cg_velocity_res(VelArgs A)
+{
+    const Dom &d = A.d;
+    const int P = d.P, NX = d.NX, NY = d.NY;
+    const Range R{A.i0, A.j0, A.i1 - A.i0, (A.i1 - A.i0) * (A.j1 - A.j0)};
+    const double EPS = 1e-14;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = q < R.n;
+    int i = A.i0, j = A.j0;
+    if (on) R.ij(q, i, j);
+    const int comp = A.comp;
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    double r = 0.0, dg = 1.0, ft = 0.0, x = 0.0, z = 0.0;
+    double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;   // viscosities of the x+, x-, y+, y- faces
+    ptrdiff_t off[4];
+    double mul[4];
+    double v[2];
+    v[0] = 0.0;
+    if (on) {
+        dg = vel_diag(d, comp, A.rho, A.mu, i, j, A.iRe, A.alpha_dt) + EPS;
+        const double *__restrict__ mu = A.mu;
+        if (comp == 0) {
+            ft = 0.5 * (AT_(A.rho, i, j) + AT_(A.rho, i - 1, j)) / A.alpha_dt;
+            m0 = AT_(mu, i, j);
+            m1 = AT_(mu, i - 1, j);
+            m2 = harm(avg2(AT_(mu, i - 1, j + 1), AT_(mu, i, j + 1)), avg2(AT_(mu, i - 1, j), AT_(mu, i, j)));
+            m3 = harm(avg2(AT_(mu, i - 1, j), AT_(mu, i, j)), avg2(AT_(mu, i - 1, j - 1), AT_(mu, i, j - 1)));
+        } else {
+            ft = 0.5 * (AT_(A.rho, i, j) + AT_(A.rho, i, j - 1)) / A.alpha_dt;
+            m0 = harm(avg2(AT_(mu, i + 1, j - 1), AT_(mu, i + 1, j)), avg2(AT_(mu, i, j - 1), AT_(mu, i, j)));
+            m1 = harm(avg2(AT_(mu, i, j - 1), AT_(mu, i, j)), avg2(AT_(mu, i - 1, j - 1), AT_(mu, i - 1, j)));
+            m2 = AT_(mu, i, j);
+            m3 = AT_(mu, i, j - 1);
+        }
+        const double ad = vel_op(d, comp, A.rho, A.mu, i, j, A.iRe, A.alpha_dt, [&](int a, int b) { return AT_(A.x, a, b); });
+        x = AT_(A.x, i, j);
+        r = AT_(A.rhs, i, j) - ad;
+        z = r / dg;
+        v[0] = r * z;
+        AT_(A.z, i, j) = z;
+        const int di[4] = {1, -1, 0, 0}, dj[4] = {0, 0, 1, -1};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            int si, sj;
+            src_of(A.mcg, NX, NY, i + di[k], j + dj[k], si, sj, mul[k]);
+            if (si < A.i0 || si >= A.i1 || sj < A.j0 || sj >= A.j1) mul[k] = 0.0;
+            off[k] = mul[k] == 0.0 ? (ptrdiff_t)j * P + i : (ptrdiff_t)sj * P + si;
+        }
+    }
+    double one[1] = {v[0]};
+    if (!grid_exchange<1, true>(sl, one)) return;
+    double rz = one[0], RMS = 0.0, beta = 0.0, dc = 0.0, dn[4] = {0.0, 0.0, 0.0, 0.0};
+    int iters = 0;
+    while (iters < A.maxit) {
+        iters++;
+        double ad = 0.0;
+        one[0] = 0.0;
+        if (on) {
+            dc = z + beta * dc;
+            double f[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) dn[k] = __ldcg(A.z + off[k]) + beta * dn[k];
+#pragma unroll
+            for (int k = 0; k < 4; k++) f[k] = mul[k] == 0.0 ? 0.0 : mul[k] * dn[k];
+            // vel_op_w at the cell
+            const double Ax = ft * dc;
+            double op = 0.0;
+            if (comp == 0) {
+                const double fxp = m0 * (f[0] - dc) * d.m.idx_u[i], fxm = m1 * (dc - f[1]) * d.m.idx_u[i - 1];
+                const double fyp = m2 * (f[2] - dc) * d.m.idy_c[j], fym = m3 * (dc - f[3]) * d.m.idy_c[j - 1];
+                op += A.iRe * u_cv_x_div(d, i, fxp, fxm);
+                op += A.iRe * (fyp - fym) * d.m.idy_v[j];
+                op += axisym_ur_term(d, i, A.iRe * 0.5 * (m0 + m1), dc);
+            } else {
+                const double fxp = m0 * (f[0] - dc) * d.m.idx_c[i], fxm = m1 * (dc - f[1]) * d.m.idx_c[i - 1];
+                const double fyp = m2 * (f[2] - dc) * d.m.idy_v[j], fym = m3 * (dc - f[3]) * d.m.idy_v[j - 1];
+                op += A.iRe * v_cv_x_div(d, i, fxp, fxm);
+                op += A.iRe * (fyp - fym) * d.m.idy_c[j - 1];
+            }
+            ad = Ax - op;
+            one[0] = dc * ad;
+        }
+        if (!grid_exchange<1, false>(sl, one)) return;
+        const double alpha = rz / (one[0] + A.step_eps);
+        v[0] = v[1] = 0.0;
+        if (on) {
+            x += alpha * dc;
+            r = r - alpha * ad;
+            z = r / dg;
+            AT_(A.z, i, j) = z;
+            v[0] = r * r / dg;
+            v[1] = r * r;
+        }
+        if (!grid_exchange<2, true>(sl, v)) return;
+        RMS = sqrt(A.in_tot * v[1]);
+        if (RMS < A.tol) break;
+        beta = v[0] / (rz + A.step_eps);
+        rz = v[0];
+    }
+    if (on) AT_(A.x, i, j) = x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->vel_iters[comp] = iters; A.scal->vel_rms[comp] = RMS; }
+}
+
+// ---------------------------------------------------------------------------
 // Velocity_solve_cg (Eulerian/lsolver/msolve_cg.c:525-722): Jacobi PCG with
 // the RMS residual stop, one velocity component.
 // ---------------------------------------------------------------------------
@@ -400,38 +612,117 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
 // variable-density Poisson operator, absolute stop on sqrt(r.M^-1 r), mean
 // removed at the end.
 //
-// FW (the context's solve): the operator's face weights 2 / (rho_P + rho_N)
-// are computed once, in the set-up phase, into the planes A.bx / A.by, so an
-// iteration multiplies instead of dividing four times per cell; without FW
-// (the no-allocation entry point, which has no room for the planes) they are
-// computed from rho at every application.  The pressure ghost rules copy
-// with weight 1 (psolve_cg.c:374-460: Neumann copies, periodic wrap) and
-// leave the solve range [0, NX-2] x [0, NY-2] unmapped, so a neighbour's
-// source differs from it only at the four ends of the axes: those sources
-// are read once from the maps and the stencil is gathered without branches.
-// The FW form also uses counting grid barriers (grid_barrier_counted; the
-// host zeroes the counter before the launch).  DEFER: the update
-// phi += alpha d of an iteration is applied in the next iteration's direction
-// pass, which reads d at the cell anyway (the same operands and operation,
-// one pass later; before the mean removal after the last iteration), so the
-// update pass reads three planes instead of five.  U1: cells per loop trip
-// of the direction pass (the update pass takes two), their loads issued
-// before either cell's stores.  Measured per iteration on B200 (the same
-// results bit for bit in every form): 1024x1024 31.7 us for the plain form
-// (without FW), 20.8 us for FW with DEFER and U1 = 1, which the context
-// uses; 2048x2048 154 and 96.6 us; 256x512 10.7 and 8.2 us.  At 64
-// registers (two 512-thread blocks per SM) U1 = 2 with DEFER loses loads in
-// flight and ran 16% slower at 2048x2048.  PAIR (k_cg_pressure_fwp): both
-// passes over pairs of neighbouring cells with 16-byte accesses, for ranges
-// of at least two cells per resident thread (the context picks it by size):
-// 2048x2048 94.0 -> 86.9 us, 1024x1024 20.7 -> 19.9 us.
+// One cell per thread (cg_pressure_resident): ranges of at most one cell per
+// resident thread (151 552 cells on a B200), the context's and the
+// no-allocation entry point's.  Bound by the latency of the two grid-wide
+// sums; per iteration 241x482 12.1 -> 7.7 us, 48x96 7.0 -> 2.4 us.
+//
+// Larger ranges (cg_pressure): the operator's face weights 2 / (rho_P +
+// rho_N) are computed once, in the set-up phase, into the planes A.bx / A.by,
+// so an iteration multiplies instead of dividing four times per cell.  The
+// pressure ghost rules copy with weight 1 (psolve_cg.c:374-460: Neumann
+// copies, periodic wrap) and leave the solve range [0, NX-2] x [0, NY-2]
+// unmapped, so a neighbour's source differs from it only at the four ends of
+// the axes: those sources are read once from the maps and the stencil is
+// gathered without branches.  The update phi += alpha d of an iteration is
+// applied in the next iteration's direction pass, which reads d at the cell
+// anyway (the same operands and operation, one pass later; before the mean
+// removal after the last iteration), so the update pass reads three planes
+// instead of five.  Measured per iteration on B200 without the planes and the
+// deferred update 31.7 us at 1024x1024 and 154 us at 2048x2048, with them
+// 20.8 and 96.6 us; two cells per trip of the direction pass ran 16% slower
+// at 2048x2048 (64 registers, loads in flight lost).  PAIR (k_cg_pressure_fwp):
+// both passes over pairs of neighbouring cells with 16-byte accesses, for
+// ranges of at least two cells per resident thread (the context picks it by
+// size): 2048x2048 94.0 -> 86.9 us, 1024x1024 20.7 -> 19.9 us.
 // ---------------------------------------------------------------------------
-template <bool FW, bool DEFER, int U1, bool PAIR>
+__device__ __forceinline__ void cg_pressure_resident(const PresArgs &A, const Range &R)
+{
+    const Dom &d = A.d;
+    const int P = d.P, NX = d.NX, NY = d.NY;
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = q < R.n;
+    int i = 0, j = 0;
+    if (on) R.ij(q, i, j);
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    double r = 0.0, m = 0.0, z = 0.0, ph = 0.0, rw = 1.0;
+    double cxm = 0.0, cxp = 0.0, cym = 0.0, cyp = 0.0;
+    const ptrdiff_t cC = (ptrdiff_t)j * P + i;
+    ptrdiff_t cE = cC, cW = cC, cN = cC, cS = cC;
+    double s[1] = {0.0};
+    if (on) {
+        // sources of the neighbours under the pressure ghost rules
+        cW = (ptrdiff_t)j * P + (i > 0 ? i - 1 : A.mp.x.src[NG - 1]);
+        cE = (ptrdiff_t)j * P + (i < NX - 2 ? i + 1 : A.mp.x.src[NX - 1 + NG]);
+        cS = (ptrdiff_t)(j > 0 ? j - 1 : A.mp.y.src[NG - 1]) * P + i;
+        cN = (ptrdiff_t)(j < NY - 2 ? j + 1 : A.mp.y.src[NY - 1 + NG]) * P + i;
+        const double *__restrict__ rho = A.rho;
+        const double r0 = rho[cC];
+        const double bxp = 2.0 / (r0 + rho[cC + 1]), bxm = 2.0 / (r0 + rho[cC - 1]);
+        const double byp = 2.0 / (r0 + rho[cC + P]), bym = 2.0 / (r0 + rho[cC - P]);
+        face_coeffs(d, i, bxm, bxp, bym, byp, cxm, cxp, cym, cyp);
+        rw = row_weight(d, i);
+        const double ad = pressure_op(d, rho, i, j, [&](int a, int b) { return remap(A.mp, A.phi, P, NX, NY, a, b); });
+        // the axisymmetric right-hand side carries the row weight r_c of the
+        // operator (psolve_hypre.c:184-200)
+        r = (d.axisym ? A.rhs[cC] * d.m.r_c[i] : A.rhs[cC]) - ad;
+        m = A.M[cC];
+        ph = A.phi[cC];
+        z = r * m;
+        A.z[cC] = z;
+        s[0] = r * z;
+    }
+    if (!grid_exchange<1, true>(sl, s)) return;
+    double gamma = s[0], gamma_new = 0.0, beta = 0.0;
+    if (sqrt(gamma) < A.tol) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = 0; A.scal->p_res = sqrt(gamma); }
+        return;
+    }
+    double dc = 0.0, dE = 0.0, dW = 0.0, dN = 0.0, dS = 0.0;
+    int iters;
+    for (iters = 1; iters <= A.maxit; iters++) {
+        double ad = 0.0;
+        s[0] = 0.0;
+        if (on) {
+            const double zE = __ldcg(A.z + cE), zW = __ldcg(A.z + cW), zN = __ldcg(A.z + cN), zS = __ldcg(A.z + cS);
+            dc = z + beta * dc;
+            dE = zE + beta * dE;
+            dW = zW + beta * dW;
+            dN = zN + beta * dN;
+            dS = zS + beta * dS;
+            const double val = cxp * (dE - dc) - cxm * (dc - dW) + cyp * (dN - dc) - cym * (dc - dS);
+            ad = rw * val;
+            s[0] = dc * ad;
+        }
+        if (!grid_exchange<1, false>(sl, s)) return;
+        const double alpha = gamma / (s[0] + 1e-30);
+        s[0] = 0.0;
+        if (on) {
+            r = r - alpha * ad;
+            z = r * m;
+            A.z[cC] = z;
+            ph += alpha * dc;
+            s[0] = r * z;
+        }
+        if (!grid_exchange<1, true>(sl, s)) return;
+        gamma_new = s[0];
+        if (sqrt(gamma_new) < A.tol) break;
+        beta = gamma_new / (gamma + 1e-30);
+        gamma = gamma_new;
+    }
+    // remove the mean (every face Neumann or periodic), psolve_cg.c:255-279
+    s[0] = on ? ph : 0.0;
+    if (!grid_exchange<1, false>(sl, s)) return;
+    if (on) A.phi[cC] = ph - s[0] / (double)R.n;
+    if (iters > A.maxit) iters = A.maxit;
+    if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = iters; A.scal->p_res = sqrt(gamma_new); }
+}
+
+template <bool PAIR>
 __device__ __forceinline__ void cg_pressure(const PresArgs &A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
-    const GridSync gs{A.scal, gridDim.x};
     const Range R{0, 0, NX - 1, (NX - 1) * (NY - 1)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     double *part0 = A.partials, *part1 = A.partials + gridDim.x, *part2 = A.partials + 2 * gridDim.x;
@@ -442,13 +733,16 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     const double *__restrict__ bx = A.bx;
     const double *__restrict__ by = A.by;
     CountedSync cs{A.scal, 0};
-    auto barrier = [&]() { return FW ? cs.sync() : grid_barrier(gs); };
+    if (!PAIR && R.n <= nth) {   // one cell per thread
+        cg_pressure_resident(A, R);
+        return;
+    }
 
     double sg = 0.0;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);
-        if (FW) pressure_face_weights(d, rho, A.bx, A.by, i, j);
+        pressure_face_weights(d, rho, A.bx, A.by, i, j);
         double ad = pressure_op(d, rho, i, j, [&](int a, int b) { return remap(A.mp, A.phi, P, NX, NY, a, b); });
         // the axisymmetric right-hand side carries the row weight r_c of the
         // operator (psolve_hypre.c:184-200)
@@ -460,7 +754,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         sg += rv * z;
     }
     put_partial(part0, sg);
-    if (!barrier()) return;
+    if (!cs.sync()) return;
     double gamma = grid_total(part0), gamma_new = 0.0, beta = 0.0;
     if (sqrt(gamma) < A.tol) {
         if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = 0; A.scal->p_res = sqrt(gamma); }
@@ -488,16 +782,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
             vn = zp[cN] + bt * dold[cN];
             vs = zp[cS] + bt * dold[cS];
         }
-        double bxm, bxp, bym, byp;
-        if (FW) {
-            bxm = bx[cC - 1]; bxp = bx[cC]; bym = by[cC - P]; byp = by[cC];
-        } else {
-            const double r0 = rho[cC];
-            bxp = 2.0 / (r0 + rho[cC + 1]);
-            bxm = 2.0 / (r0 + rho[cC - 1]);
-            byp = 2.0 / (r0 + rho[cC + P]);
-            bym = 2.0 / (r0 + rho[cC - P]);
-        }
+        const double bxm = bx[cC - 1], bxp = bx[cC], bym = by[cC - P], byp = by[cC];
         double cxm, cxp, cym, cyp;
         face_coeffs(d, i, bxm, bxp, bym, byp, cxm, cxp, cym, cyp);
         const double val = cxp * (ve - vc) - cxm * (vc - vw) + cyp * (vn - vc) - cym * (vc - vs);
@@ -545,7 +830,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         const double ad1 = row_weight(d, i1) *
                            (cxp * (ve - vc.y) - cxm * (vc.y - vc.x) + cyp * (vn.y - vc.y) - cym * (vc.y - vs.y));
         if (has1) {
-            if (DEFER && !first) {
+            if (!first) {
                 const double2 ph = ld2(A.phi + r);
                 st2(A.phi + r, ph.x + al * oc.x, ph.y + al * oc.y);
             }
@@ -554,7 +839,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
             sdad += vc.x * ad0;
             sdad += vc.y * ad1;
         } else {
-            if (DEFER && !first) A.phi[r] = A.phi[r] + al * oc.x;
+            if (!first) A.phi[r] = A.phi[r] + al * oc.x;
             if (!first) dn[r] = vc.x;
             A.Ad[r] = ad0;
             sdad += vc.x * ad0;
@@ -581,50 +866,33 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
 
     double *dcur = A.dir, *dnxt = A.dir2;
     bool first = true;
-    double alpha = 0.0;   // FW: the step of the update phi += alpha d_cur still to be applied
+    double alpha = 0.0;   // the step of the update phi += alpha d_cur still to be applied
     int iters;
     for (iters = 1; iters <= A.maxit; iters++) {
         // d = z + beta d (z = M r), Ad with the pressure ghost update of d;
-        // FW: phi += alpha d_old from the previous iteration at the cell
+        // phi += alpha d_old from the previous iteration at the cell
         double sdad = 0.0;
         const double bt = beta, al = alpha;
         const double *dold = dcur;
         if (PAIR)
             for (int p = tid; p < Np; p += nth) direction_pair(p, first, A.z, dold, dnxt, bt, al, sdad);
         else
-        for (int q = tid; q < R.n; q += U1 * nth) {
-            const int q1 = q + nth;
-            const bool two = U1 == 2 && q1 < R.n;
-            double dv0, ad0, dv1 = 0.0, ad1 = 0.0;
-            direction(q, first, A.z, dold, bt, dv0, ad0);
-            if (two) direction(q1, first, A.z, dold, bt, dv1, ad1);
+        for (int q = tid; q < R.n; q += nth) {
+            double dv, ad;
+            direction(q, first, A.z, dold, bt, dv, ad);
             int i, j;
             R.ij(q, i, j);
-            double ph0 = 0.0, do0 = 0.0, ph1 = 0.0, do1 = 0.0;
-            if (DEFER && !first) {
-                ph0 = AT_(A.phi, i, j); do0 = AT_(dold, i, j);
-                if (two) {
-                    int i1, j1;
-                    R.ij(q1, i1, j1);
-                    ph1 = AT_(A.phi, i1, j1); do1 = AT_(dold, i1, j1);
-                }
-            }
-            if (!first) AT_(dnxt, i, j) = dv0;
-            AT_(A.Ad, i, j) = ad0;
-            if (DEFER && !first) AT_(A.phi, i, j) = ph0 + al * do0;
-            sdad += dv0 * ad0;
-            if (two) {
-                R.ij(q1, i, j);
-                if (!first) AT_(dnxt, i, j) = dv1;
-                AT_(A.Ad, i, j) = ad1;
-                if (DEFER && !first) AT_(A.phi, i, j) = ph1 + al * do1;
-                sdad += dv1 * ad1;
-            }
+            double ph0 = 0.0, do0 = 0.0;
+            if (!first) { ph0 = AT_(A.phi, i, j); do0 = AT_(dold, i, j); }
+            if (!first) AT_(dnxt, i, j) = dv;
+            AT_(A.Ad, i, j) = ad;
+            if (!first) AT_(A.phi, i, j) = ph0 + al * do0;
+            sdad += dv * ad;
         }
         if (!first) { double *t = dcur; dcur = dnxt; dnxt = t; }
         first = false;
         put_partial(part1, sdad);
-        if (!barrier()) return;
+        if (!cs.sync()) return;
         alpha = gamma / (grid_total(part1) + 1e-30);
         double sgn = 0.0;
         if (PAIR)
@@ -635,41 +903,36 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
             const bool two = q1 < R.n;
             int i0, j0, i1 = 0, j1 = 0;
             R.ij(q, i0, j0);
-            double ph0 = 0.0, dc0 = 0.0, ph1 = 0.0, dc1 = 0.0;
-            if (!DEFER) { ph0 = AT_(A.phi, i0, j0); dc0 = AT_(dcur, i0, j0); }
             double r0 = AT_(A.res, i0, j0), a0 = AT_(A.Ad, i0, j0), m0 = AT_(A.M, i0, j0);
             double r1 = 0.0, a1 = 0.0, m1 = 0.0;
             if (two) {
                 R.ij(q1, i1, j1);
-                if (!DEFER) { ph1 = AT_(A.phi, i1, j1); dc1 = AT_(dcur, i1, j1); }
                 r1 = AT_(A.res, i1, j1); a1 = AT_(A.Ad, i1, j1); m1 = AT_(A.M, i1, j1);
             }
             {
                 const double rv = r0 - alpha * a0, z = rv * m0;
-                if (!DEFER) AT_(A.phi, i0, j0) = ph0 + alpha * dc0;
                 AT_(A.res, i0, j0) = rv;
                 AT_(A.z, i0, j0) = z;
                 sgn += rv * z;
             }
             if (two) {
                 const double rv = r1 - alpha * a1, z = rv * m1;
-                if (!DEFER) AT_(A.phi, i1, j1) = ph1 + alpha * dc1;
                 AT_(A.res, i1, j1) = rv;
                 AT_(A.z, i1, j1) = z;
                 sgn += rv * z;
             }
         }
         put_partial(part2, sgn);
-        if (!barrier()) return;
+        if (!cs.sync()) return;
         gamma_new = grid_total(part2);
         if (sqrt(gamma_new) < A.tol) break;
         beta = gamma_new / (gamma + 1e-30);
         gamma = gamma_new;
     }
-    // remove the mean (every face Neumann or periodic), psolve_cg.c:255-279;
-    // FW: after the last iteration's pending update
+    // remove the mean (every face Neumann or periodic), psolve_cg.c:255-279,
+    // after the last iteration's pending update
     double ssum = 0.0;
-    const bool pending = DEFER && !first;
+    const bool pending = !first;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);
@@ -677,7 +940,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         ssum += AT_(A.phi, i, j);
     }
     put_partial(part0, ssum);
-    if (!barrier()) return;
+    if (!cs.sync()) return;
     double avg = grid_total(part0) / (double)R.n;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
@@ -688,8 +951,12 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = iters; A.scal->p_res = sqrt(gamma_new); }
 }
 
-__global__ void __launch_bounds__(512) k_cg_pressure(PresArgs A) { cg_pressure<false, false, 2, false>(A); }
-__global__ void __launch_bounds__(512, 2) k_cg_pressure_fw(PresArgs A) { cg_pressure<true, true, 1, false>(A); }
-__global__ void __launch_bounds__(512, 2) k_cg_pressure_fwp(PresArgs A) { cg_pressure<true, true, 1, true>(A); }
+// the no-allocation entry point's solve: at most one cell per resident thread
+__global__ void __launch_bounds__(512) k_cg_pressure(PresArgs A)
+{
+    cg_pressure_resident(A, Range{0, 0, A.d.NX - 1, (A.d.NX - 1) * (A.d.NY - 1)});
+}
+__global__ void __launch_bounds__(512, 2) k_cg_pressure_fw(PresArgs A) { cg_pressure<false>(A); }
+__global__ void __launch_bounds__(512, 2) k_cg_pressure_fwp(PresArgs A) { cg_pressure<true>(A); }
 
 }  // namespace pvof

@@ -107,8 +107,6 @@ struct DevScalars {
     double cnn_ms[2];   // mean squares of the network's rhs and phi_prev inputs
     double mass;
     int error;          // non-zero: a grid barrier gave up (see pvof_cg.cu)
-    unsigned bar_count; // grid barrier state
-    unsigned bar_gen;
     unsigned long long bar_arrivals;   // arrivals at the counting grid barrier, zeroed before each launch
 };
 
@@ -151,7 +149,7 @@ struct Ctx {
     int *map_src_mem;
     double *map_mul_mem;
     BcMap maps[BK_COUNT];
-    double *partials;        // per-block partial sums (3 per block)
+    double *partials;        // per-block partial sums (SLOT_DOUBLES per block)
     DevScalars *scal;        // device scalars
     DevScalars *scal_host;   // pinned host mirror
     double *host_plane;      // pinned staging plane for uploads/downloads

@@ -37,6 +37,11 @@ struct VelArgs {
     double *ft = nullptr, *mc = nullptr;   // time-term and corner-viscosity planes (k_cg_velocity)
 };
 
+// doubles per block (and one more) of the partial sums: four sums of the
+// grid-stride solvers, or two buffers of two-value exchange slots (two words
+// per value) of the one-cell-per-thread ones
+constexpr size_t SLOT_DOUBLES = 8;
+
 struct PresArgs {
     Dom d;
     BcMap mp;              // Pressure_apply_BCs + exchange
@@ -47,7 +52,7 @@ struct PresArgs {
     int maxit;
     double *partials;
     DevScalars *scal;
-    double *bx = nullptr, *by = nullptr;   // face-weight planes (k_cg_pressure_fw)
+    double *bx = nullptr, *by = nullptr;   // face-weight planes (ranges of more than one cell per thread)
 };
 
 // spectral-preconditioned pressure PCG (pvof_spec.cu)
@@ -266,6 +271,7 @@ __global__ void k_fft_inverse(Dom d, int N, int logN, const double *hc, double *
 
 __global__ void k_cg_biharmonic(BihArgs A);
 __global__ void k_cg_velocity(VelArgs A);
+__global__ void k_cg_velocity_res(VelArgs A);
 __global__ void k_cg_pressure(PresArgs A);
 __global__ void k_cg_pressure_fw(PresArgs A);
 __global__ void k_cg_pressure_fwp(PresArgs A);

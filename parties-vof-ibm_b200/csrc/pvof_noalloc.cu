@@ -30,13 +30,13 @@ namespace pvof {
 constexpr size_t NOALLOC_PLANE_MAX = 72000;
 constexpr int NOALLOC_AXIS_MAX = 1024;
 constexpr int NOALLOC_THREADS = 512;
-constexpr int NOALLOC_MAX_BLOCKS = 8 * 160;
+constexpr int NOALLOC_MAX_BLOCKS = (int)((NOALLOC_PLANE_MAX + NOALLOC_THREADS - 1) / NOALLOC_THREADS);
 constexpr size_t NOALLOC_AXIS_LEN = NOALLOC_AXIS_MAX + 1 + 2 * NG;  // entries of a per-axis table
 
 // layout of the scratch array, in doubles
 constexpr size_t NA_PLANES = 6;  // M, res, dir, dir2, z, Ad
 constexpr size_t NA_OFF_PART = NA_PLANES * NOALLOC_PLANE_MAX;
-constexpr size_t NA_OFF_SCAL = NA_OFF_PART + 4 * (size_t)NOALLOC_MAX_BLOCKS;
+constexpr size_t NA_OFF_SCAL = NA_OFF_PART + SLOT_DOUBLES * (size_t)(NOALLOC_MAX_BLOCKS + 1);
 constexpr size_t NA_SCAL_LEN = (sizeof(DevScalars) + sizeof(double) - 1) / sizeof(double);
 constexpr size_t NA_OFF_METRIC = NA_OFF_SCAL + NA_SCAL_LEN;
 constexpr size_t NA_NMETRIC = 6;  // idx_c, idy_c, r_u, r_c, inv_r_c, zeros
@@ -235,8 +235,11 @@ extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const 
     A.partials = base + NA_OFF_PART;
     A.scal = scal;
     const int n = (NX - 1) * (NY - 1);
-    int nb = (n + NOALLOC_THREADS - 1) / NOALLOC_THREADS;
-    if (nb > sc.coop_blocks) nb = sc.coop_blocks;
+    const int nb = (n + NOALLOC_THREADS - 1) / NOALLOC_THREADS;   // one cell per thread: at most 141 blocks
+    if (nb > sc.coop_blocks) return na_err(PVOF_ECUDA, "the solver's blocks do not fit on the device at once");
+    // the solver's exchange slots start from epoch zero
+    if (cudaMemsetAsync(base + NA_OFF_PART, 0, SLOT_DOUBLES * (size_t)(nb + 1) * sizeof(double), st) != cudaSuccess)
+        return na_err(PVOF_ECUDA, "scratch set-up failed");
     void *args[] = {&A};
     if (cudaLaunchCooperativeKernel((const void *)k_cg_pressure, dim3((unsigned)nb), dim3(NOALLOC_THREADS), args, 0, st) !=
         cudaSuccess)
