@@ -1036,6 +1036,7 @@ int read_scalars(pvof_ctx *c)
         if (c->spec_s) CK(cudaMemsetAsync(c->spec_s, 0, sizeof(SpecScal), c->stream));
         CK(cudaStreamSynchronize(c->stream));
         return set_err(PVOF_ECUDA, code == 4 ? "advection tile load timed out"
+                                   : code == 5 ? "cluster solver: an exchange between its blocks timed out"
                                    : code == 3 ? "cluster solver: a slab edge outside the owner's boundary rows"
                                               : code == 2 ? "solver grid barrier timed out (spectral pressure solve)"
                                                           : "solver grid barrier timed out (grid-wide solver)");
