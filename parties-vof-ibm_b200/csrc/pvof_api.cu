@@ -858,7 +858,7 @@ int p_set_rhs(pvof_ctx *c, bool warm = false)
         const int rc = pvof_cnn_forward(c->cnn_params, c->cnn_bf16, c->cnn_x, c->cnn_y, c->dom.NY - 1, c->dom.NX - 1,
                                         c->cnn_work, c->stream);
         if (rc != PVOF_OK) return set_err(rc, "network forward pass");
-        c->launches += 7;
+        c->launches += 6;
         const int n = (c->dom.NX - 1) * (c->dom.NY - 1);
         const unsigned nb = 148;
         double *e = S(c, SC_P_D2);   // free until the solve starts

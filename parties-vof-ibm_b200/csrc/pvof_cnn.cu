@@ -16,14 +16,13 @@
 // training target t = (phi - phi_prev) / rms(phi_prev).
 //
 // Kernels: the four hidden 32 -> 32 layers run on the tensor cores
-// (k_conv_umma: tcgen05.mma implicit GEMM, BF16 activations and weights, FP32
-// accumulation in tensor memory), forward and input gradient, and their
-// weight gradients (k_conv_wgrad_umma, the pixels as the GEMM's K); the first
-// (3 -> 32) and last (32 -> 1) layers, too narrow for an MMA tile, are a
-// shared-memory tiled direct convolution on the FP32 pipes (one thread per
-// pixel, all output channels in registers); the input gradient is the same
-// convolution with the taps flipped and the channels swapped, the weight
-// gradient per-block partial sums; then the mean-square loss, Adam, and the
+// (k_conv_umma: tcgen05.mma on tiles staged once in shared memory, BF16
+// activations and weights, FP32 accumulation in tensor memory), forward and
+// input gradient, and their weight gradients (k_wgrad_umma, the pixels as the
+// GEMM's K); the first (3 -> 32) and last (32 -> 1) layers, too narrow for an
+// MMA tile, run on the FP32 pipes (k_conv3x3, k_conv_last, and k_last_back and
+// k_first_wgrad backwards).  Weight gradients are per-CTA partial sums that
+// one kernel adds for all layers; then the mean-square loss, Adam, and the
 // input assembly with the two root mean squares.
 #include <cuda_bf16.h>
 #include <cstdint>
@@ -86,35 +85,49 @@ __global__ void __launch_bounds__(CNN_TILE * CNN_TILE) k_conv3x3(const float *__
 // ---------------------------------------------------------------------------
 // 32 -> 32 channel 3x3 convolutions on the tensor cores (tcgen05, kind::f16)
 // ---------------------------------------------------------------------------
-// An implicit GEMM D[p][co] = sum_k A[p][k] B[co][k] over k = tap * 32 + ci
-// (288 = 18 MMAs of K = 16): one CTA of 128 threads takes 128 consecutive
-// pixels of the flattened H x W plane (the MMA's M = 128, N = 32).  Every
-// thread gathers its pixel's im2col row, rounded to BF16, into shared memory,
-// the CTA the layer's BF16 weights; both in the K-major canonical layout
-// without swizzle (core matrices of 8 rows x 16 bytes: rows 16 bytes apart,
-// the two K halves of an MMA 128 bytes apart, groups of 8 rows 256 bytes
-// apart).  One thread issues the 18 MMAs into a 128 x 32 FP32 accumulator in
-// tensor memory and commits them to an mbarrier; each warp then reads its 32
-// rows (pixels) back with tcgen05.ld and writes the 32 channels, plus the
-// bias and the ReLU.  The input-gradient convolution of the same layers is
-// this kernel with the flipped, transposed weights.
-constexpr int UM_M = 128;                          // pixels per CTA (MMA M)
+// A CTA takes a tile of TH rows x TW <= 128 pixels of the plane and stages it
+// with its one-pixel halo in shared memory once, rounded to BF16: 16-byte
+// units of 8 channels of one pixel, [row][group of 8 channels][pixel], with
+// TP = TW + 2 pixels a row.  Read as a matrix without swizzle (core matrices
+// of 8 x 16 bytes) that layout is both
+//   K-major, rows = pixels, K = channels (8-pixel groups 128 bytes apart,
+//     channel groups 16 TP bytes apart): A of the forward and input-gradient
+//     convolutions, and
+//   MN-major, rows = channels, K = pixels (channel groups 16 TP bytes apart,
+//     8-pixel groups 128 bytes apart), four rows of the tile one more run of
+//     channel groups: both operands of the weight gradient,
+// and a tap (dy, dx) of the convolution is only another start address, so no
+// im2col copy is made (it was read and stored nine times per pixel before).
+//
+// k_conv_umma: D[pixel][co] over K = tap * 32 + ci, per tile row one 128 x 32
+// FP32 accumulator in tensor memory and 18 MMAs of K = 16 in tap order.  One
+// thread issues them all and commits to an mbarrier; the warps read the
+// accumulators back and write the 32 channels with the bias and the ReLU
+// (forward) or through the ReLU mask of the layer below (input gradient, the
+// same convolution with the flipped, transposed weights).
+// Bound by the FP32 planes in HBM (256 MB per layer at 1000x1000): forward
+// 383 -> 130 us, input gradient with its mask 480 -> 158 us.
+constexpr int UM_M = 128;                          // pixels of an accumulator (MMA M)
 constexpr int UM_N = 32;                           // output channels (MMA N)
 constexpr int UM_KSTEPS = 9 * CNN_CMAX / 16;       // 18 MMAs of K = 16
-constexpr int UM_A_STEP = UM_M * 16 * 2;           // bytes of A per MMA: 4096
 constexpr int UM_B_STEP = UM_N * 16 * 2;           // bytes of B per MMA: 1024
-constexpr size_t UM_SMEM = (size_t)UM_KSTEPS * (UM_A_STEP + UM_B_STEP) + 1024;   // + alignment slack
+constexpr int UM_B_BYTES = UM_KSTEPS * UM_B_STEP;
+constexpr int UM_THREADS = 256;
 constexpr long long UM_WAIT_LIMIT = 1LL << 26;     // bounded wait on the MMAs' mbarrier
 
 // tcgen05.mma instruction descriptor: D F32 (bits 4-5 = 1), A and B BF16
-// (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 at bits
+// (bits 7-9, 10-12 = 1), A / B MN-major at bits 15 / 16, N >> 3 at bits
 // 17-22, M >> 4 at bits 24-28
-constexpr uint32_t UM_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(UM_N >> 3) << 17) |
-                              ((uint32_t)(UM_M >> 4) << 24);
+__host__ __device__ constexpr uint32_t um_idesc(int n, int mn_major)
+{
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)mn_major << 15) | ((uint32_t)mn_major << 16) |
+           ((uint32_t)(n >> 3) << 17) | ((uint32_t)(UM_M >> 4) << 24);
+}
 
-// shared-memory matrix descriptor of a K-major operand without swizzle:
-// start address, leading (K) and stride (8-row group) byte offsets, each in
-// 16-byte units; version 1 at bit 46; layout type 0 (no swizzle) at bits 61-63
+// shared-memory matrix descriptor without swizzle: start address, leading and
+// stride byte offsets, each in 16-byte units (K-major: the K halves and the
+// 8-row groups; MN-major: the 8-deep K groups and the 8-channel groups);
+// version 1 at bit 46; layout type 0 (no swizzle) at bits 61-63
 __device__ __forceinline__ uint64_t um_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo)
 {
     return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
@@ -127,356 +140,507 @@ __device__ __forceinline__ uint32_t um_pack(float a, float b)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-__global__ void __launch_bounds__(UM_M) k_conv_umma(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ w,
-                                                    const float *__restrict__ b, float *__restrict__ out, int H, int W,
-                                                    int relu, int *__restrict__ err)
-{
-    extern __shared__ unsigned char um_raw[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tmem_holder;
-    unsigned char *As = reinterpret_cast<unsigned char *>(((uintptr_t)um_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char *Bs = As + UM_KSTEPS * UM_A_STEP;
-    const int t = threadIdx.x, warp = t >> 5;
-    const long long plane = (long long)H * W;
-    const long long p = (long long)blockIdx.x * UM_M + t;
-    const bool live = p < plane;
-    const int y = live ? (int)(p / W) : 0, x = live ? (int)(p % W) : 0;
-    const uint32_t mbar_a = (uint32_t)__cvta_generic_to_shared(&mbar);
+__device__ __forceinline__ uint32_t um_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-    if (warp == 0) {   // 32 columns of tensor memory: the 128 x 32 FP32 accumulator
-        const uint32_t holder = (uint32_t)__cvta_generic_to_shared(&tmem_holder);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 32;" ::"r"(holder) : "memory");
+template <int COLS>
+__device__ __forceinline__ void um_begin(uint32_t *holder, uint64_t *mbar)
+{
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(um_smem(holder)), "n"(COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a) : "memory");
+    if (threadIdx.x == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(um_smem(mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // A: the pixel's im2col row, 16 input channels of one tap per MMA
-#pragma unroll 1
-    for (int s = 0; s < UM_KSTEPS; s++) {
-        const int tap = s >> 1, c0 = (s & 1) * 16;
-        const int xx = x + tap % 3 - 1, yy = y + tap / 3 - 1;
-        const bool ok = live && xx >= 0 && xx < W && yy >= 0 && yy < H;
-        const size_t at = ok ? (size_t)c0 * (size_t)plane + (size_t)yy * W + xx : 0;
-        uint32_t pk[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const float v0 = ok ? in[at + (size_t)(2 * e) * (size_t)plane] : 0.0f;
-            const float v1 = ok ? in[at + (size_t)(2 * e + 1) * (size_t)plane] : 0.0f;
-            pk[e] = um_pack(v0, v1);
-        }
-        unsigned char *row = As + s * UM_A_STEP + (t >> 3) * 256 + (t & 7) * 16;
-        *reinterpret_cast<uint4 *>(row) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-        *reinterpret_cast<uint4 *>(row + 128) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
-    }
-    // B: w[co][ci][tap] as rows co of K = tap * 32 + ci, 16-byte chunks (step, co, half)
-    for (int q = t; q < UM_KSTEPS * UM_N * 2; q += UM_M) {
-        const int s = q >> 6, co = (q >> 1) & 31, half = q & 1;
-        const int tap = s >> 1, c0 = (s & 1) * 16 + half * 8;
-        uint16_t v[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-            const __nv_bfloat16 wv = w[(co * CNN_CMAX + c0 + e) * 9 + tap];
-            v[e] = *reinterpret_cast<const uint16_t *>(&wv);
-        }
-        unsigned char *dst = Bs + s * UM_B_STEP + (co >> 3) * 256 + half * 128 + (co & 7) * 16;
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0] | ((uint32_t)v[1] << 16), v[2] | ((uint32_t)v[3] << 16),
-                                                     v[4] | ((uint32_t)v[5] << 16), v[6] | ((uint32_t)v[7] << 16));
-    }
-    // the generic-proxy stores above become visible to the tensor cores' async proxy
+}
+
+template <int COLS>
+__device__ __forceinline__ void um_end(uint32_t tmem)
+{
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(COLS) : "memory");
+}
+
+// the CTA's generic-proxy stores become visible to the tensor cores' async proxy
+__device__ __forceinline__ void um_publish()
+{
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_holder;
-    if (t == 0) {
-        const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(As), b0 = (uint32_t)__cvta_generic_to_shared(Bs);
-#pragma unroll 1
-        for (int s = 0; s < UM_KSTEPS; s++) {
-            const uint64_t ad = um_desc(a0 + s * UM_A_STEP, 128, 256), bd = um_desc(b0 + s * UM_B_STEP, 128, 256);
-            const uint32_t acc = s > 0 ? 1u : 0u;
-            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                         ::"r"(tmem), "l"(ad), "l"(bd), "r"(UM_IDESC), "r"(acc) : "memory");
-        }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_a)
-                     : "memory");
-    }
-    // bounded wait for the MMAs (phase 0 of the mbarrier)
+}
+
+__device__ __forceinline__ void um_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc)
+                 : "memory");
+}
+
+__device__ __forceinline__ void um_commit(uint64_t *mbar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(um_smem(mbar)) : "memory");
+}
+
+// bounded wait of the whole CTA for the committed MMAs; 0 if it gave up
+__device__ __forceinline__ int um_wait(uint64_t *mbar, uint32_t parity)
+{
     int done = 0;
     for (long long it = 0; it < UM_WAIT_LIMIT && !done; it++) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(mbar_a), "r"(0u) : "memory");
+                     "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(um_smem(mbar)), "r"(parity) : "memory");
         done = (int)ok;
     }
     done = __syncthreads_and(done);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (done) {
-        uint32_t r[32];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                     "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
-                     "%30, %31}, [%32];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                       "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                       "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-                       "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                       "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                     : "r"(taddr)
-                     : "memory");
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (live) {
+    return done;
+}
+
+__device__ __forceinline__ void um_read32(uint32_t taddr, uint32_t (&r)[32])
+{
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                 "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
+                 "%30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
+                   "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
+                   "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
+                   "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr)
+                 : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// strips of a row of W pixels: at most 128 each, a multiple of 16 wide (the
+// weight gradient's K = 16 pixels stay within a row)
+__host__ __device__ inline int um_strips(int W) { return (W + UM_M - 1) / UM_M; }
+__host__ __device__ inline int um_width(int W)
+{
+    const int n = um_strips(W), w = (W + n - 1) / n;
+    return (w + 15) / 16 * 16;
+}
+
+// `rows` rows of `width` pixels from (x0, y0) of the 32 planes of `in`, zero
+// outside the plane, as 16-byte units [row][channel group][pixel] at dst; a
+// warp takes one channel group, neighbouring lanes neighbouring pixels.  sum:
+// the FP32 sums of the warp's 8 channels over the staged pixels, if not null.
+__device__ __forceinline__ void um_stage(const float *__restrict__ in, int H, int W, int x0, int y0, int rows, int width,
+                                         unsigned char *dst, float *sum)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cg = warp & 3;
+    const size_t plane = (size_t)H * W;
+    const float *src = in + (size_t)(8 * cg) * plane;
+    const int n = rows * width, step = UM_THREADS / 4;
+    constexpr int U = 4;   // units in flight per thread: 32 loads before the first is used
+    for (int q0 = (warp >> 2) * 32 + lane; q0 < n; q0 += U * step) {
+        float v[U][8];
 #pragma unroll
-            for (int co = 0; co < UM_N; co++) {
-                float v = __uint_as_float(r[co]) + (b ? b[co] : 0.0f);
-                if (relu && v < 0.0f) v = 0.0f;
-                out[(size_t)co * (size_t)plane + (size_t)p] = v;
+        for (int u = 0; u < U; u++) {
+            const int q = q0 + u * step, r = (int)((unsigned)q / (unsigned)width);
+            const int y = y0 + r, x = x0 + q - r * width;
+            const bool ok = q < n && y >= 0 && y < H && x >= 0 && x < W;
+            const float *p = src + (ok ? (size_t)y * W + x : 0);
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[u][e] = ok ? p[(size_t)e * plane] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int q = q0 + u * step, r = (int)((unsigned)q / (unsigned)width);
+            if (q < n)
+                *reinterpret_cast<uint4 *>(dst + ((size_t)(r * 4 + cg) * width + (q - r * width)) * 16) =
+                    make_uint4(um_pack(v[u][0], v[u][1]), um_pack(v[u][2], v[u][3]), um_pack(v[u][4], v[u][5]),
+                               um_pack(v[u][6], v[u][7]));
+            if (sum)
+#pragma unroll
+                for (int e = 0; e < 8; e++) sum[e] += v[u][e];
+        }
+    }
+}
+
+template <int TH>
+constexpr size_t um_conv_smem(int TP)
+{
+    return (size_t)(TH + 2) * 4 * TP * 16 + 16 * UM_M + UM_B_BYTES;   // the last rows' 128-pixel reads run past the tile
+}
+
+template <int TH, bool DGRAD>
+__global__ void __launch_bounds__(UM_THREADS) k_conv_umma(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ w,
+                                                          const float *__restrict__ b, float *__restrict__ out,
+                                                          const float *__restrict__ mask, int H, int W, int relu,
+                                                          int *__restrict__ err)
+{
+    extern __shared__ __align__(128) unsigned char um_raw[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tmem_holder;
+    constexpr int COLS = TH * UM_N;
+    const int TW = um_width(W), TP = TW + 2, ns = um_strips(W);
+    const int x0 = (int)(blockIdx.x % ns) * TW, y0 = (int)(blockIdx.x / ns) * TH;
+    unsigned char *Bs = um_raw, *As = um_raw + UM_B_BYTES;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    um_begin<COLS>(&tmem_holder, &mbar);
+    // B: rows of the output channel, K = tap * 32 + input channel, 16-byte
+    // chunks (step, row, half), written as 4-byte words in their order in
+    // shared memory; the input gradient's weights are w flipped and
+    // transposed
+    for (int q = t; q < UM_B_BYTES / 4; q += UM_THREADS) {
+        const int s = q >> 8, n = (q >> 6 & 3) * 8 + (q >> 2 & 7), ci = (s & 1) * 16 + (q >> 5 & 1) * 8 + (q & 3) * 2;
+        const int tap = DGRAD ? 8 - (s >> 1) : s >> 1;
+        __nv_bfloat162 v;   // w[c0][c1][tap]
+        v.x = DGRAD ? w[(ci * CNN_CMAX + n) * 9 + tap] : w[(n * CNN_CMAX + ci) * 9 + tap];
+        v.y = DGRAD ? w[((ci + 1) * CNN_CMAX + n) * 9 + tap] : w[(n * CNN_CMAX + ci + 1) * 9 + tap];
+        reinterpret_cast<__nv_bfloat162 *>(Bs)[q] = v;
+    }
+    um_stage(in, H, W, x0 - 1, y0 - 1, TH + 2, TP, As, nullptr);
+    um_publish();
+    const uint32_t tmem = tmem_holder;
+    if (t == 0) {
+        const uint32_t a0 = um_smem(As), b0 = um_smem(Bs);
+#pragma unroll 1
+        for (int r = 0; r < TH; r++)
+#pragma unroll 1
+            for (int s = 0; s < UM_KSTEPS; s++) {
+                const int tap = s >> 1, dy = tap / 3, dx = tap - 3 * dy;
+                const uint32_t a = a0 + (uint32_t)((((r + dy) * 4 + 2 * (s & 1)) * TP + dx) * 16);
+                um_mma(tmem + (uint32_t)(r * UM_N), um_desc(a, (uint32_t)TP * 16, 128), um_desc(b0 + s * UM_B_STEP, 128, 256),
+                       um_idesc(UM_N, 0), s > 0 ? 1u : 0u);
+            }
+        um_commit(&mbar);
+    }
+    if (um_wait(&mbar, 0)) {
+        const size_t plane = (size_t)H * W;
+        const int px = (warp & 3) * 32 + lane, x = x0 + px;
+#pragma unroll 1
+        for (int r = warp >> 2; r < TH; r += UM_THREADS / 128) {
+            const int y = y0 + r;
+            const bool live = px < TW && x < W && y < H;
+            const size_t p = live ? (size_t)y * W + x : 0;
+            uint32_t pass = 0xffffffffu;   // the ReLU mask of the layer below, by channel
+            if (DGRAD && live) {
+                pass = 0;
+#pragma unroll
+                for (int co = 0; co < UM_N; co++) pass |= (mask[(size_t)co * plane + p] > 0.0f ? 1u : 0u) << co;
+            }
+            uint32_t v[32];
+            um_read32(tmem + (uint32_t)(r * UM_N) + ((uint32_t)((warp & 3) * 32) << 16), v);
+            if (live) {
+#pragma unroll
+                for (int co = 0; co < UM_N; co++) {
+                    float f = __uint_as_float(v[co]);
+                    if (DGRAD) {
+                        if (!(pass >> co & 1u)) f = 0.0f;
+                    } else {
+                        f += b ? b[co] : 0.0f;
+                        if (relu && f < 0.0f) f = 0.0f;
+                    }
+                    out[(size_t)co * plane + p] = f;
+                }
             }
         }
     } else if (t == 0) {
         atomicExch(err, 1);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 32;" ::"r"(tmem) : "memory");
+    um_end<COLS>(tmem);
 }
 
-// Weight gradient of a 32 -> 32 layer on the tensor cores: the GEMM
-// D[m][co] = sum_p A[m][p] G[co][p] over the pixels, m = tap * 32 + ci
-// (288 rows in three M = 128 tiles, the last one padded with zeros),
-// A[m][p] = in[ci][p + tap] and G the layer's output gradient, both rounded to
-// BF16.  Each CTA takes 128-pixel chunks of the plane (grid-stride), gathers
-// them into shared memory in the K-major canonical layout (K = pixels),
-// issues 3 x 8 MMAs per chunk into three 128 x 32 FP32 accumulators in tensor
-// memory, and at the end writes its 288 x 32 partial sums; k_wgrad_reduce adds
-// the CTAs' partials in a fixed order.
-constexpr int UW_PIX = 128;                                   // pixels per chunk
-constexpr int UW_TILES = 3;                                   // M tiles of 128 (288 rows)
-constexpr int UW_A_TILE_STEP = UM_M * 16 * 2;                 // bytes of one tile for one MMA: 4096
-constexpr int UW_A_BYTES = UW_TILES * (UW_PIX / 16) * UW_A_TILE_STEP;   // 98304
-constexpr int UW_B_BYTES = (UW_PIX / 16) * UM_B_STEP;         // 8192
-constexpr size_t UW_SMEM = (size_t)UW_A_BYTES + UW_B_BYTES + 1024;
+// Weight and bias gradient of a 32 -> 32 layer: dw[co][ci][tap] = sum_p
+// in[ci][p + tap] g[co][p], the pixels as K.  Per pair of output rows and 16
+// pixels one MMA for each dx: M = four input rows x 32 ci, N = the two rows x
+// 32 co, so every vertical tap of the pair is a block of the 128 x 64
+// accumulator (input row minus output row).  A CTA walks its tiles of UW_TH
+// rows, the three accumulators staying in tensor memory, and writes its
+// partial sums in dw's order, the bias sums (FP32, of the unrounded g) behind
+// them; k_grad_reduce adds the CTAs' partials in a fixed order.  Two CTAs per
+// SM, one staging while the other multiplies.  1000x1000: 1645 -> 102 us.
+constexpr int UW_TH = 4;
+constexpr int UW_COLS = 256;                                  // 3 x 64 accumulator columns
+constexpr int GRAD32 = 9 * CNN_CMAX * CNN_CMAX + CNN_CMAX;    // weights and biases of a hidden layer
 
-__global__ void __launch_bounds__(UM_M) k_conv_wgrad_umma(const float *__restrict__ in, const float *__restrict__ g,
-                                                          int H, int W, float *__restrict__ partial,
-                                                          int *__restrict__ err)
+size_t um_wgrad_smem(int TW)   // the staged tiles, later the sums of the nine taps
 {
-    extern __shared__ unsigned char uw_raw[];
+    const size_t tiles = (size_t)((UW_TH + 2) * 4 * (TW + 2) + UW_TH * 4 * TW) * 16, sums = sizeof(float) * 9 * CNN_CMAX * CNN_CMAX;
+    return tiles > sums ? tiles : sums;
+}
+
+__global__ void __launch_bounds__(UM_THREADS) k_wgrad_umma(const float *__restrict__ in, const float *__restrict__ g, int H,
+                                                           int W, float *__restrict__ partial, int *__restrict__ err)
+{
+    extern __shared__ __align__(128) unsigned char um_raw[];
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_holder;
-    unsigned char *As = reinterpret_cast<unsigned char *>(((uintptr_t)uw_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char *Bs = As + UW_A_BYTES;
-    const int t = threadIdx.x, warp = t >> 5;
-    const long long plane = (long long)H * W;
-    const long long nchunk = (plane + UW_PIX - 1) / UW_PIX;
-    const uint32_t mbar_a = (uint32_t)__cvta_generic_to_shared(&mbar);
-    if (warp == 0) {   // 3 x 32 columns: the three accumulators (allocated as 128)
-        const uint32_t holder = (uint32_t)__cvta_generic_to_shared(&tmem_holder);
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(holder) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar_a) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    // rows 288..383 (rows 32..127 of the last tile: row groups 4..15) stay zero
-    for (int q = t; q < (UW_PIX / 16) * 12 * 2 * 8; q += UM_M) {   // steps x 12 row groups x 2 halves x 8 rows
-        const int s = q / 192, rest = q % 192;
-        unsigned char *dst = As + (2 * (UW_PIX / 16) + s) * UW_A_TILE_STEP + (4 + rest / 16) * 256 +
-                             ((rest / 8) & 1) * 128 + (rest & 7) * 16;
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_holder;
-    const uint32_t a0 = (uint32_t)__cvta_generic_to_shared(As), b0 = (uint32_t)__cvta_generic_to_shared(Bs);
-    int ok_all = 1;
-    uint32_t phase = 0;
-    bool first = true;
-#pragma unroll 1
-    for (long long c = blockIdx.x; c < nchunk; c += gridDim.x) {
-        const long long p0 = c * UW_PIX;
-        // A: 288 rows (tap, ci) x 128 pixels, 16-byte chunks of 8 pixels
-#pragma unroll 1
-        for (int q = t; q < 288 * (UW_PIX / 8); q += UM_M) {
-            const int m = q / (UW_PIX / 8), k8 = q % (UW_PIX / 8);
-            const int tap = m >> 5, ci = m & 31, dx = tap % 3 - 1, dy = tap / 3 - 1;
-            uint32_t pk[4];
+    __shared__ float bsum[UM_THREADS / 32][8];
+    const int TW = um_width(W), TP = TW + 2, ns = um_strips(W), ntile = ns * ((H + UW_TH - 1) / UW_TH);
+    unsigned char *As = um_raw, *Gs = um_raw + (UW_TH + 2) * 4 * TP * 16;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    um_begin<UW_COLS>(&tmem_holder, &mbar);
+    float bs[8];
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                float v[2];
+    for (int e = 0; e < 8; e++) bs[e] = 0.0f;
+    uint32_t phase = 0, tmem = 0;
+    int ok = 1;
+#pragma unroll 1
+    for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
+        const int x0 = (tile % ns) * TW, y0 = (tile / ns) * UW_TH;
+        um_stage(in, H, W, x0 - 1, y0 - 1, UW_TH + 2, TP, As, nullptr);
+        um_stage(g, H, W, x0, y0, UW_TH, TW, Gs, bs);
+        um_publish();
+        tmem = tmem_holder;
+        if (t == 0) {
+            const uint32_t a0 = um_smem(As), g0 = um_smem(Gs);
+#pragma unroll 1
+            for (int pr = 0; pr < UW_TH / 2; pr++)
+#pragma unroll 1
+                for (int k = 0; k < TW / 16; k++)
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const long long pp = p0 + k8 * 8 + 2 * e + h;
-                    v[h] = 0.0f;
-                    if (pp < plane) {
-                        const int y = (int)(pp / W) + dy, x = (int)(pp % W) + dx;
-                        if (x >= 0 && x < W && y >= 0 && y < H) v[h] = in[(size_t)ci * plane + (size_t)y * W + x];
+                    for (int dx = 0; dx < 3; dx++)
+                        um_mma(tmem + (uint32_t)(dx * 64),
+                               um_desc(a0 + (uint32_t)((2 * pr * 4 * TP + 16 * k + dx) * 16), 128, (uint32_t)TP * 16),
+                               um_desc(g0 + (uint32_t)((2 * pr * 4 * TW + 16 * k) * 16), 128, (uint32_t)TW * 16),
+                               um_idesc(64, 1), (tile != (int)blockIdx.x || pr > 0 || k > 0) ? 1u : 0u);
+            um_commit(&mbar);
+        }
+        ok = um_wait(&mbar, phase);   // the MMAs read the staged tiles
+        phase ^= 1u;
+    }
+    float *out = partial + (size_t)blockIdx.x * GRAD32;
+    if (ok) {
+        // lanes ra * 32 + ci (input row ra), columns dx * 64 + rb * 32 + co
+        // (output row rb): vertical tap dy = ra - rb in 0..2; the two output
+        // rows' blocks are added through shared memory
+        float *acc = reinterpret_cast<float *>(um_raw);   // [tap][ci][co], co rotated by ci against bank conflicts
+#pragma unroll 1
+        for (int rb = 0; rb < 2; rb++) {
+            if (warp < 4 && warp - rb >= 0 && warp - rb < 3)
+#pragma unroll 1
+                for (int dx = 0; dx < 3; dx++) {
+                    uint32_t v[32];
+                    um_read32(tmem + (uint32_t)(dx * 64 + rb * 32) + ((uint32_t)(warp * 32) << 16), v);
+                    float *p = acc + (((warp - rb) * 3 + dx) * CNN_CMAX + lane) * CNN_CMAX;
+#pragma unroll
+                    for (int co = 0; co < CNN_CMAX; co++) {
+                        const int q = (co + lane) & 31;
+                        p[q] = rb == 0 ? __uint_as_float(v[co]) : p[q] + __uint_as_float(v[co]);
                     }
                 }
-                pk[e] = um_pack(v[0], v[1]);
-            }
-            const int tile = m >> 7, row = m & 127, s = k8 >> 1, half = k8 & 1;
-            unsigned char *dst = As + (tile * (UW_PIX / 16) + s) * UW_A_TILE_STEP + (row >> 3) * 256 + half * 128 +
-                                 (row & 7) * 16;
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            __syncthreads();
         }
-        // B: the output gradient, 32 rows (co) x 128 pixels
-        for (int q = t; q < UM_N * (UW_PIX / 8); q += UM_M) {
-            const int co = q / (UW_PIX / 8), k8 = q % (UW_PIX / 8);
-            uint32_t pk[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const long long pp = p0 + k8 * 8 + 2 * e;
-                const float v0 = pp < plane ? g[(size_t)co * plane + (size_t)pp] : 0.0f;
-                const float v1 = pp + 1 < plane ? g[(size_t)co * plane + (size_t)pp + 1] : 0.0f;
-                pk[e] = um_pack(v0, v1);
-            }
-            const int s = k8 >> 1, half = k8 & 1;
-            unsigned char *dst = Bs + s * UM_B_STEP + (co >> 3) * 256 + half * 128 + (co & 7) * 16;
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        for (int q = t; q < 9 * CNN_CMAX * CNN_CMAX; q += UM_THREADS) {
+            const int tap = q % 9, ci = (q / 9) & 31, co = q / (9 * CNN_CMAX);
+            out[q] = acc[(tap * CNN_CMAX + ci) * CNN_CMAX + ((co + ci) & 31)];
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (t == 0) {
-#pragma unroll 1
-            for (int tile = 0; tile < UW_TILES; tile++)
-#pragma unroll 1
-                for (int s = 0; s < UW_PIX / 16; s++) {
-                    const uint64_t ad = um_desc(a0 + (tile * (UW_PIX / 16) + s) * UW_A_TILE_STEP, 128, 256);
-                    const uint64_t bd = um_desc(b0 + s * UM_B_STEP, 128, 256);
-                    const uint32_t acc = (first && s == 0) ? 0u : 1u;
-                    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                                 "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                 ::"r"(tmem + (uint32_t)(tile * UM_N)), "l"(ad), "l"(bd), "r"(UM_IDESC), "r"(acc)
-                                 : "memory");
-                }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar_a)
-                         : "memory");
-        }
-        first = false;
-        // the MMAs read the shared tiles: wait before the next chunk overwrites them
-        int done = 0;
-        for (long long it = 0; it < UM_WAIT_LIMIT && !done; it++) {
-            uint32_t okw;
-            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                         "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(okw) : "r"(mbar_a), "r"(phase) : "memory");
-            done = (int)okw;
-        }
-        phase ^= 1u;
-        ok_all = __syncthreads_and(done);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!ok_all) break;
-    }
-    if (ok_all && !first) {
-        float *out = partial + (size_t)blockIdx.x * 288 * UM_N;
-#pragma unroll 1
-        for (int tile = 0; tile < UW_TILES; tile++) {
-            uint32_t r[32];
-            const uint32_t taddr = tmem + (uint32_t)(tile * UM_N) + ((uint32_t)(warp * 32) << 16);
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
-                         "%12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, "
-                         "%30, %31}, [%32];"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                           "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                           "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-                           "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-                           "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                         : "r"(taddr)
-                         : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int m = tile * UM_M + t;
-            if (m < 288)
-#pragma unroll
-                for (int co = 0; co < UM_N; co++) out[(size_t)m * UM_N + co] = __uint_as_float(r[co]);
-        }
-    } else if (t == 0 && !ok_all) {
+    } else if (t == 0) {
         atomicExch(err, 1);
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem) : "memory");
-}
-
-// dw[co][ci][tap] += sum over the CTAs (in order) of partial[cta][tap * 32 + ci][co]
-__global__ void k_wgrad_reduce(const float *__restrict__ partial, int nparts, float *__restrict__ dw)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;   // q = m * 32 + co
-    if (q >= 288 * UM_N) return;
-    float s = 0.0f;
-    for (int c = 0; c < nparts; c++) s += partial[(size_t)c * 288 * UM_N + q];
-    const int m = q / UM_N, co = q % UM_N, tap = m >> 5, ci = m & 31;
-    dw[(co * CNN_CMAX + ci) * 9 + tap] += s;
-}
-
-// the weights of the input-gradient convolution: wt[ci][co][8 - tap] = w[co][ci][tap]
-__global__ void k_conv_transpose_weights(const __nv_bfloat16 *__restrict__ w, __nv_bfloat16 *__restrict__ wt,
-                                         int cout, int cin)
-{
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= cout * cin * 9) return;
-    const int co = q / (cin * 9), ci = (q / 9) % cin, t = q % 9;
-    wt[(ci * cout + co) * 9 + (8 - t)] = w[q];
-}
-
-// dY *= (y > 0): the ReLU of a hidden layer, backwards
-__global__ void k_relu_back(float *__restrict__ dy, const float *__restrict__ y, size_t n)
-{
-    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q < n && !(y[q] > 0.0f)) dy[q] = 0.0f;
-}
-
-// weight and bias gradients of one layer: block (co, ci) sums
-// in[ci][p + tap] * dY[co][p] over the pixels for the nine taps; block
-// (co, cin) sums dY[co][p] for the bias
-__global__ void __launch_bounds__(256) k_conv_wgrad(const float *__restrict__ in, int cin,
-                                                    const float *__restrict__ dy, int H, int W,
-                                                    float *__restrict__ dw, float *__restrict__ db)
-{
-    const int co = blockIdx.y, ci = blockIdx.x;
-    const size_t plane = (size_t)H * W;
-    const float *g = dy + co * plane;
-    float acc[9];
 #pragma unroll
-    for (int t = 0; t < 9; t++) acc[t] = 0.0f;
-    const bool bias = ci == cin;
-    for (size_t p = threadIdx.x; p < plane; p += blockDim.x) {
-        const float gv = g[p];
-        if (gv == 0.0f) continue;
-        if (bias) {
-            acc[0] += gv;
-            continue;
+    for (int e = 0; e < 8; e++) {
+        for (int o = 16; o > 0; o >>= 1) bs[e] += __shfl_down_sync(0xffffffffu, bs[e], o);
+        if (lane == 0) bsum[warp][e] = bs[e];
+    }
+    __syncthreads();
+    if (t < CNN_CMAX) out[9 * CNN_CMAX * CNN_CMAX + t] = bsum[t >> 3][t & 7] + bsum[4 + (t >> 3)][t & 7];
+    um_end<UW_COLS>(tmem_holder);
+}
+
+// ---------------------------------------------------------------------------
+// the narrow layers (3 -> 32 and 32 -> 1) on the FP32 pipes
+// ---------------------------------------------------------------------------
+
+// the last layer forward: 32 planes to one, every thread LAST_ROWS pixels of a
+// column (4, or 1 where that leaves SMs idle: 64x64 19.6 -> 13.8 us), its accumulators in k_conv3x3's order (ci, then tap).  y2: a second
+// copy of the output, if not null.  1000x1000: 181 -> 113 us (read of 128 MB).
+template <int LAST_ROWS>
+__global__ void __launch_bounds__(256) k_conv_last(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ w,
+                                                   const float *__restrict__ b, float *__restrict__ y1,
+                                                   float *__restrict__ y2, int H, int W)
+{
+    __shared__ float ws[CNN_CMAX * 9];
+    for (int q = threadIdx.x; q < CNN_CMAX * 9; q += 256) ws[q] = __bfloat162float(w[q]);
+    __syncthreads();
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * LAST_ROWS;
+    if (x >= W || y0 >= H) return;
+    const size_t plane = (size_t)H * W;
+    float acc[LAST_ROWS];
+#pragma unroll
+    for (int k = 0; k < LAST_ROWS; k++) acc[k] = b[0];
+#pragma unroll(LAST_ROWS == 1 ? 4 : 2)
+    for (int ci = 0; ci < CNN_CMAX; ci++) {
+        const float *p = in + (size_t)ci * plane;
+        float v[LAST_ROWS + 2][3];
+#pragma unroll
+        for (int r = 0; r < LAST_ROWS + 2; r++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const int yy = y0 + r - 1, xx = x + c - 1;
+                v[r][c] = (yy >= 0 && yy < H && xx >= 0 && xx < W) ? p[(size_t)yy * W + xx] : 0.0f;
+            }
+#pragma unroll
+        for (int tp = 0; tp < 9; tp++) {
+            const float wv = ws[ci * 9 + tp];
+#pragma unroll
+            for (int k = 0; k < LAST_ROWS; k++) acc[k] += v[k + tp / 3][tp % 3] * wv;
         }
-        const int i = (int)(p % W), j = (int)(p / W);
-        const float *x = in + ci * plane;
+    }
+#pragma unroll
+    for (int k = 0; k < LAST_ROWS; k++)
+        if (y0 + k < H) {
+            const size_t q = (size_t)(y0 + k) * W + x;
+            y1[q] = acc[k];
+            if (y2) y2[q] = acc[k];
+        }
+}
+
+// the last layer backward in one pass over its 32 input planes: the gradient
+// at its input through that layer's ReLU (gout) and the partial weight and
+// bias gradients.  A pixel needs the nine values of dy around it for both; a
+// warp takes 8 channels, so a thread holds 72 weight-gradient sums.  Partials
+// [block][w (32 x 9), b].  1000x1000: 4.7 ms in three kernels -> 135 us.
+constexpr int GRAD_LAST = CNN_CMAX * 9 + 1;
+constexpr int LB_THREADS = 256;
+__global__ void __launch_bounds__(LB_THREADS) k_last_back(const float *__restrict__ act, const float *__restrict__ dy,
+                                                          const __nv_bfloat16 *__restrict__ w, int H, int W,
+                                                          float *__restrict__ gout, float *__restrict__ partial)
+{
+    __shared__ float ws[CNN_CMAX * 9];
+    __shared__ float red[LB_THREADS / 32][73];
+    for (int q = threadIdx.x; q < CNN_CMAX * 9; q += LB_THREADS) ws[q] = __bfloat162float(w[q]);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cg = warp & 3;
+    const int plane = H * W;
+    float acc[8][9], bacc = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 8; e++)
+#pragma unroll
+        for (int t = 0; t < 9; t++) acc[e][t] = 0.0f;
+    for (int p = (blockIdx.x * 2 + (warp >> 2)) * 32 + lane; p < plane; p += gridDim.x * 64) {
+        const int x = p % W, y = p / W;
+        float n[9];
 #pragma unroll
         for (int t = 0; t < 9; t++) {
-            const int a = i + t % 3 - 1, c = j + t / 3 - 1;
-            if (a >= 0 && a < W && c >= 0 && c < H) acc[t] += x[(size_t)c * W + a] * gv;
+            const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
+            n[t] = (xx >= 0 && xx < W && yy >= 0 && yy < H) ? dy[(size_t)yy * W + xx] : 0.0f;
         }
-    }
-    __shared__ float red[8][9];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        bacc += n[4];
 #pragma unroll
-    for (int t = 0; t < 9; t++) {
-        float v = acc[t];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) red[warp][t] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 9) {
-        float v = 0.0f;
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) v += red[q][threadIdx.x];
-        if (bias) {
-            if (threadIdx.x == 0) db[co] += v;
-        } else {
-            dw[(co * cin + ci) * 9 + threadIdx.x] += v;
+        for (int e = 0; e < 8; e++) {
+            const int ci = 8 * cg + e;
+            const size_t q = (size_t)ci * plane + p;
+            const float a = act[q];
+            float g = 0.0f;
+#pragma unroll
+            for (int t = 0; t < 9; t++) g += n[t] * ws[ci * 9 + 8 - t];
+            gout[q] = a > 0.0f ? g : 0.0f;
+#pragma unroll
+            for (int t = 0; t < 9; t++) acc[e][t] += a * n[8 - t];
         }
+    }
+#pragma unroll
+    for (int e = 0; e < 8; e++)
+#pragma unroll
+        for (int t = 0; t < 9; t++) {
+            float v = acc[e][t];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) red[warp][e * 9 + t] = v;
+        }
+    for (int o = 16; o > 0; o >>= 1) bacc += __shfl_down_sync(0xffffffffu, bacc, o);
+    if (lane == 0) red[warp][72] = bacc;
+    __syncthreads();
+    float *out = partial + (size_t)blockIdx.x * GRAD_LAST;
+    for (int q = threadIdx.x; q < GRAD_LAST; q += LB_THREADS)
+        out[q] = q < CNN_CMAX * 9 ? red[q / 72][q % 72] + red[4 + q / 72][q % 72] : red[0][72] + red[4][72];
+}
+
+// the first layer's weight and bias gradient: a warp takes FW_CO of the 32
+// output channels, so a thread holds 54 weight sums and reads the 27 inputs
+// around its pixel (through L1, without bounds checks where the whole warp is
+// inside the plane).  Partials [block][w (32 x 3 x 9), b (32)].  1000x1000:
+// 2.3 ms -> 285 us.
+constexpr int CNN_IN = 3;
+constexpr int GRAD_FIRST = CNN_CMAX * CNN_IN * 9 + CNN_CMAX;
+constexpr int FW_CO = 2, FW_THREADS = 32 * CNN_CMAX / FW_CO;
+__global__ void __launch_bounds__(FW_THREADS) k_first_wgrad(const float *__restrict__ in, const float *__restrict__ g, int H,
+                                                            int W, float *__restrict__ partial)
+{
+    const int lane = threadIdx.x & 31, c0 = (threadIdx.x >> 5) * FW_CO;
+    const int plane = H * W;
+    float acc[FW_CO][27], bacc[FW_CO];
+#pragma unroll
+    for (int e = 0; e < FW_CO; e++) {
+        bacc[e] = 0.0f;
+#pragma unroll
+        for (int t = 0; t < 27; t++) acc[e][t] = 0.0f;
+    }
+    const int step = gridDim.x * 32, sy = step / W, sx = step - sy * W;
+    int p = blockIdx.x * 32 + lane, y = p / W, x = p - y * W;
+    for (; p - lane < plane; p += step) {
+        const bool live = p < plane;
+        float gv[FW_CO];
+#pragma unroll
+        for (int e = 0; e < FW_CO; e++) {
+            gv[e] = live ? g[(size_t)(c0 + e) * plane + p] : 0.0f;
+            bacc[e] += gv[e];
+        }
+        float v[27];
+        if (__all_sync(0xffffffffu, live && x > 0 && x < W - 1 && y > 0 && y < H - 1)) {
+#pragma unroll
+            for (int t = 0; t < 27; t++) v[t] = in[(ptrdiff_t)(t / 9) * plane + p + (ptrdiff_t)(t % 9 / 3 - 1) * W + t % 3 - 1];
+        } else {
+#pragma unroll
+            for (int t = 0; t < 27; t++) {
+                const int xx = x + t % 3 - 1, yy = y + t % 9 / 3 - 1;
+                v[t] = (live && xx >= 0 && xx < W && yy >= 0 && yy < H) ? in[(size_t)(t / 9) * plane + (size_t)yy * W + xx] : 0.0f;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < 27; t++)
+#pragma unroll
+            for (int e = 0; e < FW_CO; e++) acc[e][t] += v[t] * gv[e];
+        x += sx;
+        y += sy;
+        if (x >= W) { x -= W; y++; }
+    }
+    float *out = partial + (size_t)blockIdx.x * GRAD_FIRST;
+#pragma unroll
+    for (int e = 0; e < FW_CO; e++) {
+#pragma unroll
+        for (int t = 0; t < 27; t++) {
+            float v = acc[e][t];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) out[(c0 + e) * 27 + t] = v;
+        }
+        for (int o = 16; o > 0; o >>= 1) bacc[e] += __shfl_down_sync(0xffffffffu, bacc[e], o);
+        if (lane == 0) out[CNN_CMAX * 27 + c0 + e] = bacc[e];
+    }
+}
+
+// grad += the partials of every layer, a layer's parts added in a fixed order:
+// 8 threads per value take every 8th part each, their sums added in order
+struct GradPart {
+    const float *p;
+    int n, parts, at;   // values, parts, first index in grad
+};
+struct GradParts {
+    GradPart l[6];
+};
+__global__ void __launch_bounds__(256) k_grad_reduce(const __grid_constant__ GradParts G, float *__restrict__ grad, int total)
+{
+    __shared__ float sh[8][32];
+    const int q = blockIdx.x * 32 + (threadIdx.x & 31), s = threadIdx.x >> 5;
+    float v = 0.0f;
+    if (q < total) {
+        int l = 0;
+        while (l < 5 && q >= G.l[l + 1].at) l++;
+        const float *p = G.l[l].p + (q - G.l[l].at);
+        const int n = G.l[l].n, parts = G.l[l].parts;
+#pragma unroll 8
+        for (int c = s; c < parts; c += 8) v += p[(size_t)c * n];
+    }
+    sh[s][threadIdx.x & 31] = v;
+    __syncthreads();
+    if (s == 0 && q < total) {
+        for (int k = 1; k < 8; k++) v += sh[k][threadIdx.x & 31];
+        grad[q] += v;
     }
 }
 
@@ -525,7 +689,6 @@ struct Layer {
 };
 
 constexpr int CNN_LAYERS = 6;
-constexpr int CNN_IN = 3;
 
 void layers(Layer (&L)[CNN_LAYERS])
 {
@@ -547,73 +710,68 @@ size_t param_count()
     return L[CNN_LAYERS - 1].b + 1;
 }
 
-// activation planes kept in the work buffer: the five hidden layers' outputs
-// (32 planes each) and the output plane, then two gradient buffers of 32
-// planes, then the transposed weights of one layer
+// work buffer: the five hidden layers' outputs (32 planes each), the output
+// plane, two gradient buffers of 32 planes, and the backward pass's partial
+// sums of every layer
 __device__ int g_cnn_err;   // set when a tensor-core convolution gave up waiting for its MMAs
 
-constexpr int UW_MAX_CTAS = 296;   // tensor-core weight-gradient CTAs (two per SM of a B200)
+constexpr int GRAD_CTAS = 296;   // most blocks of a weight gradient (two per SM of a B200)
+
+int wgrad_ctas(int H, int W)   // tensor-core layers: every CTA gets a tile
+{
+    const long long n = (long long)um_strips(W) * ((H + UW_TH - 1) / UW_TH);
+    return (int)(n < GRAD_CTAS ? n : GRAD_CTAS);
+}
+int pixel_ctas(int H, int W, int per)   // narrow layers: a block takes `per` pixels a trip
+{
+    const long long n = ((long long)H * W + per - 1) / per;
+    return (int)(n < GRAD_CTAS ? n : GRAD_CTAS);
+}
 
 size_t work_floats(int H, int W)
 {
     const size_t plane = (size_t)H * W;
-    return (5 * CNN_CMAX + 1 + 2 * CNN_CMAX) * plane + CNN_CMAX * CNN_CMAX * 9 + (size_t)UW_MAX_CTAS * 288 * UM_N;
+    return (5 * CNN_CMAX + 1 + 2 * CNN_CMAX) * plane + 4 * (size_t)wgrad_ctas(H, W) * GRAD32 +
+           (size_t)pixel_ctas(H, W, 64) * GRAD_LAST + (size_t)pixel_ctas(H, W, 32) * GRAD_FIRST;
 }
 
-// weight and bias gradient of a 32 -> 32 layer: the weights on the tensor
-// cores, the bias by per-block sums
-int wgrad32(const float *in, const float *g, float *dw, float *db, int H, int W, float *partial, cudaStream_t st)
+int *cnn_error()
 {
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv_wgrad_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UW_SMEM) !=
-            cudaSuccess)
-            return -1;
-        attr = true;
-    }
     int *err = nullptr;
-    if (cudaGetSymbolAddress((void **)&err, g_cnn_err) != cudaSuccess) return -1;
-    const long long n = (long long)H * W, nchunk = (n + UW_PIX - 1) / UW_PIX;
-    const int nb = (int)(nchunk < UW_MAX_CTAS ? nchunk : UW_MAX_CTAS);   // every CTA gets a chunk
-    k_conv_wgrad_umma<<<(unsigned)nb, UM_M, UW_SMEM, st>>>(in, g, H, W, partial, err);
-    k_wgrad_reduce<<<(288 * UM_N + 255) / 256, 256, 0, st>>>(partial, nb, dw);
-    k_conv_wgrad<<<dim3(1u, (unsigned)CNN_CMAX), 256, 0, st>>>(in, 0, g, H, W, dw, db);   // bias only
+    return cudaGetSymbolAddress((void **)&err, g_cnn_err) == cudaSuccess ? err : nullptr;
+}
+
+// A hidden layer's convolution, forward (mask null) or input gradient through
+// the ReLU mask of the layer below.  Tiles of 8 rows where they fill the SMs,
+// else of 4 or 2 (more CTAs; a tile's halo rows are read again by its
+// neighbours: 10 rows for 8, 4 for 2).
+template <int TH, bool DGRAD>
+int conv32_launch(const float *in, const __nv_bfloat16 *w, const float *b, float *out, const float *mask, int H, int W, int relu,
+                  cudaStream_t st)
+{
+    const size_t sm = um_conv_smem<TH>(um_width(W) + 2);
+    int *err = cnn_error();
+    if (!err || !raise_dynamic_smem((const void *)k_conv_umma<TH, DGRAD>, sm)) return -1;
+    k_conv_umma<TH, DGRAD><<<(unsigned)(um_strips(W) * ((H + TH - 1) / TH)), UM_THREADS, sm, st>>>(in, w, b, out, mask, H, W, relu, err);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-size_t conv_smem(int cin, int cout) { return sizeof(float) * ((size_t)cin * CNN_HALO * CNN_HALO + (size_t)cout * cin * 9); }
-
-int conv(const float *in, int cin, const __nv_bfloat16 *w, const float *b, float *out, int cout, int H, int W, int relu,
-         cudaStream_t st)
+template <bool DGRAD>
+int conv32(const float *in, const __nv_bfloat16 *w, const float *b, float *out, const float *mask, int H, int W, int relu,
+           cudaStream_t st)
 {
-    if (cin == CNN_CMAX && cout == CNN_CMAX) {   // the hidden layers: tensor cores
-        static bool um_attr = false;
-        if (!um_attr) {
-            if (cudaFuncSetAttribute(k_conv_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)UM_SMEM) !=
-                cudaSuccess)
-                return -1;
-            um_attr = true;
-        }
-        int *err = nullptr;
-        if (cudaGetSymbolAddress((void **)&err, g_cnn_err) != cudaSuccess) return -1;
-        const long long n = (long long)H * W;
-        k_conv_umma<<<(unsigned)((n + UM_M - 1) / UM_M), UM_M, UM_SMEM, st>>>(in, w, b, out, H, W, relu, err);
-        return cudaGetLastError() == cudaSuccess ? 0 : -1;
-    }
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_conv3x3<CNN_CMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)conv_smem(CNN_CMAX, CNN_CMAX)) != cudaSuccess ||
-            cudaFuncSetAttribute(k_conv3x3<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)conv_smem(CNN_CMAX, 1)) != cudaSuccess)
-            return -1;
-        attr = true;
-    }
+    const long long ns = um_strips(W);
+    if (ns * (H / 8) >= 148) return conv32_launch<8, DGRAD>(in, w, b, out, mask, H, W, relu, st);
+    if (ns * (H / 4) >= 148) return conv32_launch<4, DGRAD>(in, w, b, out, mask, H, W, relu, st);
+    return conv32_launch<2, DGRAD>(in, w, b, out, mask, H, W, relu, st);
+}
+
+// the first layer, 3 -> 32 planes
+int conv_first(const float *in, const __nv_bfloat16 *w, const float *b, float *out, int H, int W, cudaStream_t st)
+{
+    const size_t sm = sizeof(float) * ((size_t)CNN_IN * CNN_HALO * CNN_HALO + (size_t)CNN_CMAX * CNN_IN * 9);
     const dim3 grd((unsigned)((W + CNN_TILE - 1) / CNN_TILE), (unsigned)((H + CNN_TILE - 1) / CNN_TILE));
-    const size_t sm = conv_smem(cin, cout);
-    if (cout == CNN_CMAX) k_conv3x3<CNN_CMAX><<<grd, CNN_TILE * CNN_TILE, sm, st>>>(in, cin, w, b, out, H, W, relu);
-    else if (cout == 1) k_conv3x3<1><<<grd, CNN_TILE * CNN_TILE, sm, st>>>(in, cin, w, b, out, H, W, relu);
-    else return -1;
+    k_conv3x3<CNN_CMAX><<<grd, CNN_TILE * CNN_TILE, sm, st>>>(in, CNN_IN, w, b, out, H, W, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -754,16 +912,19 @@ int pvof_cnn_forward(const float *params, const uint16_t *params_bf16, const flo
     layers(L);
     const size_t plane = (size_t)H * W;
     const __nv_bfloat16 *wb = reinterpret_cast<const __nv_bfloat16 *>(params_bf16);
-    const float *in = x;
-    for (int l = 0; l < CNN_LAYERS; l++) {
-        float *out = work + (size_t)l * CNN_CMAX * plane;   // layer l's output (the last: one plane)
-        if (conv(in, L[l].cin, wb + L[l].w, params + L[l].b, out, L[l].cout, H, W, l < CNN_LAYERS - 1, st))
-            return PVOF_ECUDA;
+    if (conv_first(x, wb + L[0].w, params + L[0].b, work, H, W, st)) return PVOF_ECUDA;
+    const float *in = work;
+    for (int l = 1; l < CNN_LAYERS - 1; l++) {
+        float *out = work + (size_t)l * CNN_CMAX * plane;   // layer l's output
+        if (conv32<false>(in, wb + L[l].w, params + L[l].b, out, nullptr, H, W, 1, st)) return PVOF_ECUDA;
         in = out;
     }
-    if (y && cudaMemcpyAsync(y, in, plane * sizeof(float), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return PVOF_ECUDA;
-    return PVOF_OK;
+    const Layer &Z = L[CNN_LAYERS - 1];   // the last: one plane, and y
+    float *y0 = work + (size_t)(CNN_LAYERS - 1) * CNN_CMAX * plane;
+    const unsigned gx = (unsigned)((W + 31) / 32), gy4 = (unsigned)((H + 31) / 32);
+    if (gx * gy4 >= 148) k_conv_last<4><<<dim3(gx, gy4), 256, 0, st>>>(in, wb + Z.w, params + Z.b, y0, y, H, W);
+    else k_conv_last<1><<<dim3(gx, (unsigned)((H + 7) / 8)), 256, 0, st>>>(in, wb + Z.w, params + Z.b, y0, y, H, W);
+    return cudaGetLastError() == cudaSuccess ? PVOF_OK : PVOF_ECUDA;
 }
 
 int pvof_cnn_backward(const float *params, const uint16_t *params_bf16, const float *x, const float *dy, float *grad,
@@ -777,32 +938,33 @@ int pvof_cnn_backward(const float *params, const uint16_t *params_bf16, const fl
     const size_t plane = (size_t)H * W;
     const __nv_bfloat16 *wb = reinterpret_cast<const __nv_bfloat16 *>(params_bf16);
     float *gbuf[2] = {work + (5 * CNN_CMAX + 1) * plane, work + (6 * CNN_CMAX + 1) * plane};
-    __nv_bfloat16 *wt = reinterpret_cast<__nv_bfloat16 *>(work + (7 * CNN_CMAX + 1) * plane);
-    float *partial = work + (7 * CNN_CMAX + 1) * plane + CNN_CMAX * CNN_CMAX * 9;
-    // gradient at the output of the last layer
-    if (cudaMemcpyAsync(gbuf[0], dy, plane * sizeof(float), cudaMemcpyDeviceToDevice, st) != cudaSuccess)
-        return PVOF_ECUDA;
+    float *part = work + (7 * CNN_CMAX + 1) * plane;   // every layer's partial sums, added at the end
+    GradParts G;
+    auto parts = [&](int l, int n, int ctas) {
+        float *p = part;
+        G.l[l] = GradPart{p, n, ctas, (int)L[l].w};
+        part += (size_t)n * ctas;
+        return p;
+    };
+    int *err = cnn_error();
+    const size_t wsm = um_wgrad_smem(um_width(W));
+    if (!err || !raise_dynamic_smem((const void *)k_wgrad_umma, wsm)) return PVOF_ECUDA;
+    // the last layer: its gradients and the gradient at its input, through the ReLU
+    const int last = CNN_LAYERS - 1, nl = pixel_ctas(H, W, 64);
+    k_last_back<<<(unsigned)nl, LB_THREADS, 0, st>>>(work + (size_t)(last - 1) * CNN_CMAX * plane, dy, wb + L[last].w, H, W,
+                                                    gbuf[0], parts(last, GRAD_LAST, nl));
     int cur = 0;
-    for (int l = CNN_LAYERS - 1; l >= 0; l--) {
-        const float *lin = l == 0 ? x : work + (size_t)(l - 1) * CNN_CMAX * plane;
-        float *g = gbuf[cur];
-        if (l < CNN_LAYERS - 1) {   // through this layer's ReLU
-            const size_t n = (size_t)L[l].cout * plane;
-            k_relu_back<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, work + (size_t)l * CNN_CMAX * plane, n);
-        }
-        if (L[l].cin == CNN_CMAX && L[l].cout == CNN_CMAX) {   // a tensor-core layer
-            if (wgrad32(lin, g, grad + L[l].w, grad + L[l].b, H, W, partial, st)) return PVOF_ECUDA;
-        } else {
-            k_conv_wgrad<<<dim3((unsigned)L[l].cin + 1, (unsigned)L[l].cout), 256, 0, st>>>(
-                lin, L[l].cin, g, H, W, grad + L[l].w, grad + L[l].b);
-        }
-        if (l > 0) {   // gradient at this layer's input: the flipped, transposed convolution
-            const int n = L[l].cout * L[l].cin * 9;
-            k_conv_transpose_weights<<<(n + 255) / 256, 256, 0, st>>>(wb + L[l].w, wt, L[l].cout, L[l].cin);
-            if (conv(g, L[l].cout, wt, nullptr, gbuf[1 - cur], L[l].cin, H, W, 0, st)) return PVOF_ECUDA;
-            cur = 1 - cur;
-        }
+    const int nw = wgrad_ctas(H, W);
+    for (int l = last - 1; l >= 1; l--) {   // the tensor-core layers
+        const float *lin = work + (size_t)(l - 1) * CNN_CMAX * plane;
+        k_wgrad_umma<<<(unsigned)nw, UM_THREADS, wsm, st>>>(lin, gbuf[cur], H, W, parts(l, GRAD32, nw), err);
+        if (conv32<true>(gbuf[cur], wb + L[l].w, nullptr, gbuf[1 - cur], lin, H, W, 0, st)) return PVOF_ECUDA;
+        cur = 1 - cur;
     }
+    const int nf = pixel_ctas(H, W, 32);
+    k_first_wgrad<<<(unsigned)nf, FW_THREADS, 0, st>>>(x, gbuf[cur], H, W, parts(0, GRAD_FIRST, nf));
+    const int total = (int)param_count();
+    k_grad_reduce<<<(unsigned)((total + 31) / 32), 256, 0, st>>>(G, grad, total);
     return cudaGetLastError() == cudaSuccess ? PVOF_OK : PVOF_ECUDA;
 }
 
@@ -830,8 +992,7 @@ int pvof_cnn_conv32(const float *x, const uint16_t *w_bf16, const float *b, floa
                     void *stream)
 {
     if (!x || !w_bf16 || !y || H <= 0 || W <= 0) return PVOF_EINVAL;
-    return conv(x, CNN_CMAX, reinterpret_cast<const __nv_bfloat16 *>(w_bf16), b, y, CNN_CMAX, H, W, relu,
-                (cudaStream_t)stream)
+    return conv32<false>(x, reinterpret_cast<const __nv_bfloat16 *>(w_bf16), b, y, nullptr, H, W, relu, (cudaStream_t)stream)
                ? PVOF_ECUDA
                : PVOF_OK;
 }
