@@ -189,7 +189,7 @@ struct Ctx {
     int npend;
     IbmState *ibm;           // resolved particles (null until pvof_set_particles)
     pvof3::Handle *h3;       // the 3D mode's state (PVOF_GEOM_3D); null for the 2D modes
-    double *fft_coef;        // as, ap, an (NY-1 each) and the modified wavenumbers (NX-1)
+    double *fft_coef;        // the FFT Poisson solver's tables (p_solve_fft)
     double *spec_mem;        // spectral pressure preconditioner: twiddles, block sums, reduction tables
     struct SpecScal *spec_s; // its grid barrier state
     double spec_fscale;      // dy^2 / N

@@ -264,10 +264,24 @@ __global__ void k_cnn_galerkin(Dom d, BcMap mp, const double *rho, const double 
 __global__ void k_cnn_apply(Dom d, const double *e, const double *phi_prev, const DevScalars *sc, double *phi);
 
 // constant-density Poisson solver (pvof_fft.cu)
-__global__ void k_fft_forward(Dom d, int N, int logN, const double *rhs, double *hc, double inx);
-__global__ void k_fft_tridiag(Dom d, int N, int NYp, const double *as_, const double *ap_, const double *an_,
-                              const double *mw, double *hc, double *gam);
-__global__ void k_fft_inverse(Dom d, int N, int logN, const double *hc, double *out);
+struct FftRadices {
+    int n, largest;
+    int r[16];
+};
+FftRadices fft_radices(int n);
+struct FftArgs {
+    int N, M;                     // x and y cells
+    int pairs;                    // pairs of rows per block of the x transforms
+    int cols;                     // wave numbers per block of the y solve (0: Thomas)
+    double inx;                   // 1 / N
+    const double2 *twx, *twy;     // exp(-2 pi i k / N), exp(-2 pi i k / M)
+    const double2 *wy;            // exp(-i pi k / 2M), k <= M / 2
+    const double *mw, *ly;        // -eigenvalues in x (k <= N / 2) and y (k < M)
+    FftRadices rx, ry;
+};
+// thomas: as, ap, an (M each), read when cols is 0; hat, gam: scratch planes
+cudaError_t fft_solve_launch(const Dom &d, const FftArgs &A, const double *thomas, const double *rhs, double *hat, double *gam,
+                             double *out, cudaStream_t st);
 
 __global__ void k_cg_biharmonic(BihArgs A);
 __global__ void k_cg_velocity(VelArgs A);
