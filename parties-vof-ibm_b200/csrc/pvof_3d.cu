@@ -11,6 +11,7 @@
 #include <cmath>
 #include <cstdio>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -305,217 +306,274 @@ __global__ void __launch_bounds__(256) k3p_dir(Dom3 d, const double *__restrict_
 // Thomas algorithm from host tables; the constant mode (the operator's null
 // space) gets eigenvalue 1 in units of 1/dy^2.  Spectrum layout: element
 // (kx, j, kz) at ((kz * ny + j) * H + kx), H = N/2 + 1.
+//
+// The transforms (power-of-two lengths) keep 8 points of a transform per thread
+// in registers: Stockham passes of radix 8, with a last one of 4 or 2 where the
+// length is no power of 8, exchanged through shared memory between passes only
+// (the first pass takes its inputs from global memory, the last leaves its
+// outputs in registers at the same indices).  Bound by HBM (a pass reads and
+// writes the spectrum or the box once).  256^3, B200: forward x 275 -> 66 us,
+// z 202 -> 53, inverse x 327 -> 96 (radix-2 stages two at a time in shared memory
+// before, with a square root per point and direction).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
-
-// twiddles w[q] = exp(sign 2 pi i q / n), q < n/2, into shared memory from
-// the table of exp(-2 pi i q / n) made once on the host
-__device__ __forceinline__ void fft_twiddles(double2 *w, const double2 *__restrict__ tab, int n, double sign)
+__device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
-    for (int q = threadIdx.x; q < n / 2; q += blockDim.x) {
-        const double2 v = tab[q];
-        w[q] = make_double2(v.x, sign < 0.0 ? v.y : -v.y);
-    }
+    return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+template <bool INV>
+__device__ __forceinline__ double2 crot(double2 a)   // times -i (forward) or i (inverse)
+{
+    return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
 }
 
-// in-place radix-2 transform of a[0..n) (n = 2^logn) by the nt threads of
-// one group (t = the thread's index in it); every thread of the block runs
-// the same stages, so the block barriers line up
-__device__ __forceinline__ void fft_group(double2 *a, const double2 *w, int n, int logn, int t, int nt)
+template <bool INV>
+__device__ __forceinline__ void dft4(double2 &a, double2 &b, double2 &c, double2 &d)   // in natural order, in place
 {
-    for (int q = t; q < n; q += nt) {
-        const int r = (int)(__brev((unsigned)q) >> (32 - logn));
-        if (r > q) {
-            const double2 x = a[q];
-            a[q] = a[r];
-            a[r] = x;
-        }
-    }
-    __syncthreads();
-    // two radix-2 stages per pass over shared memory: a thread takes the four
-    // elements the two stages combine (the same butterflies and twiddles as
-    // one stage at a time, so the same numbers), half the shared-memory round
-    // trips and barriers
+    const double2 s = cadd(a, c), t = csub(a, c), u = cadd(b, d), v = crot<INV>(csub(b, d));
+    a = cadd(s, u);
+    b = cadd(t, v);
+    c = csub(s, u);
+    d = csub(t, v);
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft8(double2 (&v)[8])
+{
+    const double h = 0.70710678118654752440;
+    dft4<INV>(v[0], v[2], v[4], v[6]);
+    dft4<INV>(v[1], v[3], v[5], v[7]);
+    // odd part times exp(-+ 2 pi i k / 8)
+    const double2 o1 = INV ? make_double2(h * (v[3].x - v[3].y), h * (v[3].x + v[3].y))
+                           : make_double2(h * (v[3].x + v[3].y), h * (v[3].y - v[3].x));
+    const double2 o2 = crot<INV>(v[5]);
+    const double2 o3 = INV ? make_double2(-h * (v[7].x + v[7].y), h * (v[7].x - v[7].y))
+                           : make_double2(h * (v[7].y - v[7].x), -h * (v[7].x + v[7].y));
+    const double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+    v[0] = cadd(e0, o0);
+    v[4] = csub(e0, o0);
+    v[1] = cadd(e1, o1);
+    v[5] = csub(e1, o1);
+    v[2] = cadd(e2, o2);
+    v[6] = csub(e2, o2);
+    v[3] = cadd(e3, o3);
+    v[7] = csub(e3, o3);
+}
+
+// The transform of 2^LOGN points by N / 8 threads: thread b holds points
+// b + (N / 8) k in v[k], before and after.  put / get: a point's place in
+// shared memory; sync: all threads of the transform.  tw: exp(-2 pi i k / N).
+template <int LOGN, bool INV, class Put, class Get, class Sync>
+__device__ __forceinline__ void fft_regs(double2 (&v)[8], int b, const double2 *__restrict__ tw, Put put, Get get, Sync sync)
+{
+    constexpr int N = 1 << LOGN, T = N / 8, P8 = LOGN / 3;
     int s = 1;
-    for (; s + 1 <= logn; s += 2) {
-        const int h = 1 << (s - 1), st0 = n >> s, st1 = n >> (s + 1);
-        for (int b = t; b < n / 4; b += nt) {
-            const int pos = b & (h - 1), p = ((b >> (s - 1)) << (s + 1)) + pos;
-            const double2 x0 = a[p], x1 = a[p + h], x2 = a[p + 2 * h], x3 = a[p + 3 * h];
-            const double2 w0 = w[pos * st0];
-            const double2 v1 = cmul(w0, x1), v3 = cmul(w0, x3);
-            const double2 y0 = make_double2(x0.x + v1.x, x0.y + v1.y), y1 = make_double2(x0.x - v1.x, x0.y - v1.y);
-            const double2 y2 = make_double2(x2.x + v3.x, x2.y + v3.y), y3 = make_double2(x2.x - v3.x, x2.y - v3.y);
-            const double2 u2 = cmul(w[pos * st1], y2), u3 = cmul(w[(pos + h) * st1], y3);
-            a[p] = make_double2(y0.x + u2.x, y0.y + u2.y);
-            a[p + 2 * h] = make_double2(y0.x - u2.x, y0.y - u2.y);
-            a[p + h] = make_double2(y1.x + u3.x, y1.y + u3.y);
-            a[p + 3 * h] = make_double2(y1.x - u3.x, y1.y - u3.y);
+#pragma unroll
+    for (int f = 0; f < P8; f++, s *= 8) {
+        dft8<INV>(v);
+        if (3 * (f + 1) == LOGN) return;   // the last pass: no twiddles, outputs in place
+        const int p = b / s, q = b - p * s;
+        double2 w1 = __ldg(tw + p * s), w2 = __ldg(tw + 2 * p * s), w4 = __ldg(tw + 4 * p * s);
+        if (INV) {
+            w1.y = -w1.y;
+            w2.y = -w2.y;
+            w4.y = -w4.y;
         }
-        __syncthreads();
+        const double2 w3 = cmul(w1, w2);
+        v[1] = cmul(v[1], w1);
+        v[2] = cmul(v[2], w2);
+        v[3] = cmul(v[3], w3);
+        v[4] = cmul(v[4], w4);
+        v[5] = cmul(v[5], cmul(w4, w1));
+        v[6] = cmul(v[6], cmul(w4, w2));
+        v[7] = cmul(v[7], cmul(w4, w3));
+        sync();   // the previous exchange has been read
+#pragma unroll
+        for (int k = 0; k < 8; k++) put(q + s * (8 * p + k), v[k]);
+        sync();
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = get(b + T * k);
     }
-    if (s == logn) {   // an odd number of stages: the last one alone
-        const int half = 1 << (s - 1), stride = n >> s;
-        for (int b = t; b < n / 2; b += nt) {
-            const int pos = b & (half - 1), i0 = ((b >> (s - 1)) << s) + pos, i1 = i0 + half;
-            const double2 u = a[i0], v = cmul(w[pos * stride], a[i1]);
-            a[i0] = make_double2(u.x + v.x, u.y + v.y);
-            a[i1] = make_double2(u.x - v.x, u.y - v.y);
+    if constexpr (LOGN % 3 == 2) {
+        dft4<INV>(v[0], v[2], v[4], v[6]);
+        dft4<INV>(v[1], v[3], v[5], v[7]);
+    } else if constexpr (LOGN % 3 == 1) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const double2 x = v[u], y = v[u + 4];
+            v[u] = cadd(x, y);
+            v[u + 4] = csub(x, y);
         }
-        __syncthreads();
     }
 }
 
 struct SpecDims {
     int N, logN, K, logK, ny, H;
-    int nt_x, g_x;   // x transforms: threads per pair of rows, pairs per block
-    int ch_z, nt_z;  // z transforms: columns per block, threads per column
+    int g_x;         // x transforms: pairs of rows per block
+    int ch_z;        // z transforms: columns per block
 };
+constexpr int XT = 256;   // threads per block of the x transforms
 
 // t = s r along two x rows at once (one as the real part, the other as the
 // imaginary part of a complex row), forward transform, then the two half
 // spectra separated, X_a = (Z_k + conj Z_(N-k)) / 2 and
 // X_b = (Z_k - conj Z_(N-k)) / 2i, and stored
-__global__ void __launch_bounds__(256) k3s_fwd_x(Dom3 d, SpecDims sd, const double *__restrict__ R,
-                                                 const double *__restrict__ M, double2 *__restrict__ SP,
-                                                 const double2 *__restrict__ TW, const int *gate)
+template <int LOGN>
+__global__ void __launch_bounds__(XT, 2) k3s_fwd_x(Dom3 d, SpecDims sd, const double *__restrict__ R,
+                                                   const double *__restrict__ SM, double2 *__restrict__ SP,
+                                                   const double2 *__restrict__ TW, const int *gate)
 {
-    extern __shared__ double2 sm[];
+    constexpr int N = 1 << LOGN, T = N / 8, G = XT / T, H = N / 2 + 1;
+    __shared__ double2 sm[G * (N + N / 8)];
     if (gate && *gate == 0) return;
-    double2 *w = sm, *a = sm + sd.N / 2 + (threadIdx.x / sd.nt_x) * sd.N;
-    fft_twiddles(w, TW, sd.N, -1.0);
-    const int g = threadIdx.x / sd.nt_x, t = threadIdx.x % sd.nt_x;
+    const int g = threadIdx.x / T, b = threadIdx.x % T;
+    double2 *a = sm + g * (N + N / 8);
     const long long rows = (long long)sd.K * sd.ny;
-    const long long ra = 2 * ((long long)blockIdx.x * sd.g_x + g), rb = ra + 1;   // row = k * ny + j
+    const long long ra = 2 * ((long long)blockIdx.x * G + g), rb = ra + 1;   // row = k * ny + j
     const bool la = ra < rows, lb = rb < rows;
-    const int ja = la ? (int)(ra % sd.ny) : 0, ka = la ? (int)(ra / sd.ny) : 0;
-    const int jb = lb ? (int)(rb % sd.ny) : 0, kb = lb ? (int)(rb / sd.ny) : 0;
-    for (int i = t; i < sd.N; i += sd.nt_x) {
-        double va = 0.0, vb = 0.0;
-        if (la) {
-            const long long q = at(d, i, ja, ka);
-            va = sqrt(M[q]) * R[q];
-        }
-        if (lb) {
-            const long long q = at(d, i, jb, kb);
-            vb = sqrt(M[q]) * R[q];
-        }
-        a[i] = make_double2(va, vb);
-    }
-    __syncthreads();
-    fft_group(a, w, sd.N, sd.logN, t, sd.nt_x);
-    for (int kx = t; kx < sd.H; kx += sd.nt_x) {
-        const double2 zk = a[kx], zn = a[(sd.N - kx) & (sd.N - 1)];
-        if (la) SP[ra * sd.H + kx] = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
-        if (lb) SP[rb * sd.H + kx] = make_double2(0.5 * (zk.y + zn.y), -0.5 * (zk.x - zn.x));
+    const long long qa = la ? at(d, b, (int)(ra % sd.ny), (int)(ra / sd.ny)) : 0;
+    const long long qb = lb ? at(d, b, (int)(rb % sd.ny), (int)(rb / sd.ny)) : 0;
+    double2 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        v[k] = make_double2(la ? SM[qa + T * k] * R[qa + T * k] : 0.0, lb ? SM[qb + T * k] * R[qb + T * k] : 0.0);
+    auto sync = [] { if (T <= 32) __syncwarp(); else __syncthreads(); };
+    auto put = [&](int i, double2 x) { a[i + (i >> 3)] = x; };
+    auto get = [&](int i) { return a[i + (i >> 3)]; };
+    fft_regs<LOGN, false>(v, b, TW, put, get, sync);
+    sync();
+#pragma unroll
+    for (int k = 0; k < 8; k++) put(b + T * k, v[k]);
+    sync();
+#pragma unroll
+    for (int k = 0; k <= 4; k++) {
+        const int kx = b + T * k;
+        if (kx >= H) break;
+        const double2 zk = get(kx), zn = get((N - kx) & (N - 1));
+        if (la) SP[ra * H + kx] = make_double2(0.5 * (zk.x + zn.x), 0.5 * (zk.y - zn.y));
+        if (lb) SP[rb * H + kx] = make_double2(0.5 * (zk.y + zn.y), -0.5 * (zk.x - zn.x));
     }
 }
 
-// complex transform along z of ch_z neighbouring kx columns at one j
-__global__ void __launch_bounds__(256) k3s_z(SpecDims sd, double2 *__restrict__ SP, const double2 *__restrict__ TW,
-                                             double sign, const int *gate)
+// complex transform along z of ch_z neighbouring kx columns at one j;
+// neighbouring threads take neighbouring columns
+template <int LOGK, bool INV>
+__global__ void __launch_bounds__(256) k3s_z(SpecDims sd, double2 *__restrict__ SP, const double2 *__restrict__ TW, const int *gate)
 {
-    extern __shared__ double2 sm[];
+    constexpr int K = 1 << LOGK, T = K / 8, CH = 256 / T < 32 ? 256 / T : 32;
+    __shared__ double2 sm[K * CH];
     if (gate && *gate == 0) return;
-    double2 *w = sm, *a = sm + sd.K / 2;
-    fft_twiddles(w, TW, sd.K, sign);
-    const int nchunk = (sd.H + sd.ch_z - 1) / sd.ch_z;
-    const int j = blockIdx.x / nchunk, kx0 = (blockIdx.x % nchunk) * sd.ch_z;
-    const int c = threadIdx.x / sd.nt_z, t = threadIdx.x % sd.nt_z;
-    // load: element (kz, col) of the tile at a[col * K + kz]
-    for (int e = threadIdx.x; e < sd.K * sd.ch_z; e += blockDim.x) {
-        const int kz = e / sd.ch_z, col = e % sd.ch_z, kx = kx0 + col;
-        a[col * sd.K + kz] = (kx < sd.H) ? SP[((long long)kz * sd.ny + j) * sd.H + kx] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    fft_group(a + c * sd.K, w, sd.K, sd.logK, t, sd.nt_z);
-    for (int e = threadIdx.x; e < sd.K * sd.ch_z; e += blockDim.x) {
-        const int kz = e / sd.ch_z, col = e % sd.ch_z, kx = kx0 + col;
-        if (kx < sd.H) SP[((long long)kz * sd.ny + j) * sd.H + kx] = a[col * sd.K + kz];
-    }
+    const int nchunk = (sd.H + CH - 1) / CH;
+    const int j = blockIdx.x / nchunk, c = threadIdx.x % CH, kx = (blockIdx.x % nchunk) * CH + c, b = threadIdx.x / CH;
+    const bool live = kx < sd.H;
+    const long long step = (long long)sd.ny * sd.H;
+    double2 *p = SP + (long long)b * step + (long long)j * sd.H + (live ? kx : 0);
+    double2 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = live ? p[(long long)(T * k) * step] : make_double2(0.0, 0.0);
+    fft_regs<LOGK, INV>(v, b, TW, [&](int i, double2 x) { sm[i * CH + c] = x; }, [&](int i) { return sm[i * CH + c]; },
+                        [] { __syncthreads(); });
+    if (live)
+#pragma unroll
+        for (int k = 0; k < 8; k++) p[(long long)(T * k) * step] = v[k];
 }
 
-// one tridiagonal system in y per (kx, kz): (m_j)^-1 and c'_j from the host
-// tables; the right-hand side scaled by dy^2 / (N K) (the transforms' norm)
-__global__ void __launch_bounds__(32) k3s_tri(SpecDims sd, double2 *__restrict__ SP, const double *__restrict__ CP,
-                                               const double *__restrict__ IM, double scale, const int *gate)
+// one tridiagonal system in y per (kx, kz): (m_j)^-1 from the host table (the
+// upper coefficient of the eliminated rows is its negative); the right-hand
+// side scaled by dy^2 / (N K) (the transforms' norm).  Both sweeps, and the
+// constant mode's, in runs of TU rows: a run's loads are all issued before its
+// dependent chain of updates.  Bound by HBM: the spectrum is read and written by
+// each sweep (256^3 146 us).
+__global__ void __launch_bounds__(32) k3s_tri(SpecDims sd, double2 *__restrict__ SP, const double *__restrict__ IM, double scale,
+                                               const int *gate)
 {
     if (gate && *gate == 0) return;
     const long long sys = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (sys >= (long long)sd.K * sd.H) return;
     const int kz = (int)(sys / sd.H), kx = (int)(sys % sd.H);
     const int ny = sd.ny;
+    constexpr int TU = 8;
     auto idx = [&](int j) { return ((long long)kz * ny + j) * sd.H + kx; };
+    auto load = [&](double2 (&v)[TU], int j0) {
+#pragma unroll
+        for (int u = 0; u < TU; u++)
+            if (j0 + u < ny) v[u] = SP[idx(j0 + u)];
+    };
+    auto store = [&](const double2 (&v)[TU], int j0) {
+#pragma unroll
+        for (int u = 0; u < TU; u++)
+            if (j0 + u < ny) SP[idx(j0 + u)] = v[u];
+    };
     if (kx == 0 && kz == 0) {
         // the constant mode: the mean-free part by the recurrence of rows
         // 0..ny-2 from u_0 = 0, its mean removed, plus the mean itself
-        double2 mean = make_double2(0.0, 0.0);
-        for (int j = 0; j < ny; j++) {
-            const double2 v = SP[idx(j)];
-            mean.x += v.x;
-            mean.y += v.y;
+        double2 v[TU], mean = make_double2(0.0, 0.0);
+        for (int j0 = 0; j0 < ny; j0 += TU) {
+            load(v, j0);
+#pragma unroll
+            for (int u = 0; u < TU; u++)
+                if (j0 + u < ny) mean = cadd(mean, v[u]);
         }
         mean.x *= scale / ny;
         mean.y *= scale / ny;
         double2 um = make_double2(0.0, 0.0), uc = make_double2(0.0, 0.0), su = make_double2(0.0, 0.0);
-        for (int j = 0; j < ny; j++) {
-            double2 un;
-            const double2 dj = SP[idx(j)];
-            const double2 dd = make_double2(dj.x * scale - mean.x, dj.y * scale - mean.y);
-            SP[idx(j)] = uc;
-            su.x += uc.x;
-            su.y += uc.y;
-            if (j == 0) un = make_double2(uc.x - dd.x, uc.y - dd.y);
-            else un = make_double2(2.0 * uc.x - um.x - dd.x, 2.0 * uc.y - um.y - dd.y);
-            um = uc;
-            uc = un;
+        for (int j0 = 0; j0 < ny; j0 += TU) {
+            load(v, j0);
+#pragma unroll
+            for (int u = 0; u < TU; u++)
+                if (j0 + u < ny) {
+                    const double2 dd = make_double2(v[u].x * scale - mean.x, v[u].y * scale - mean.y);
+                    const double2 un = j0 + u == 0 ? csub(uc, dd)
+                                                   : make_double2(2.0 * uc.x - um.x - dd.x, 2.0 * uc.y - um.y - dd.y);
+                    su = cadd(su, uc);
+                    v[u] = uc;
+                    um = uc;
+                    uc = un;
+                }
+            store(v, j0);
         }
         su.x /= ny;
         su.y /= ny;
-        for (int j = 0; j < ny; j++) {
-            const double2 v = SP[idx(j)];
-            SP[idx(j)] = make_double2(v.x - su.x + mean.x, v.y - su.y + mean.y);
+        for (int j0 = 0; j0 < ny; j0 += TU) {
+            load(v, j0);
+#pragma unroll
+            for (int u = 0; u < TU; u++)
+                if (j0 + u < ny) v[u] = make_double2(v[u].x - su.x + mean.x, v[u].y - su.y + mean.y);
+            store(v, j0);
         }
         return;
     }
-    // both sweeps in runs of TU rows: a run's loads are all issued before its
-    // dependent chain of updates (a thread's loads would otherwise wait one
-    // memory latency per row)
-    constexpr int TU = 8;
     double2 dp = make_double2(0.0, 0.0);
     for (int j0 = 0; j0 < ny; j0 += TU) {
         double2 v[TU];
         double m[TU];
+        load(v, j0);
 #pragma unroll
         for (int u = 0; u < TU; u++)
-            if (j0 + u < ny) {
-                v[u] = SP[idx(j0 + u)];
-                m[u] = IM[idx(j0 + u)];
-            }
+            if (j0 + u < ny) m[u] = IM[idx(j0 + u)];
 #pragma unroll
         for (int u = 0; u < TU; u++)
             if (j0 + u < ny) {
                 dp = make_double2((v[u].x * scale + dp.x) * m[u], (v[u].y * scale + dp.y) * m[u]);
                 v[u] = dp;
             }
-#pragma unroll
-        for (int u = 0; u < TU; u++)
-            if (j0 + u < ny) SP[idx(j0 + u)] = v[u];
+        store(v, j0);
     }
     double2 x = dp;   // u_{ny-1}
     for (int j1 = ny - 2; j1 >= 0; j1 -= TU) {
         double2 v[TU];
-        double c[TU];
+        double m[TU];
 #pragma unroll
         for (int u = 0; u < TU; u++)
             if (j1 - u >= 0) {
                 v[u] = SP[idx(j1 - u)];
-                c[u] = CP[idx(j1 - u)];
+                m[u] = IM[idx(j1 - u)];
             }
 #pragma unroll
         for (int u = 0; u < TU; u++)
             if (j1 - u >= 0) {
-                x = make_double2(v[u].x - c[u] * x.x, v[u].y - c[u] * x.y);
+                x = make_double2(v[u].x + m[u] * x.x, v[u].y + m[u] * x.y);
                 v[u] = x;
             }
 #pragma unroll
@@ -571,52 +629,49 @@ __device__ __forceinline__ void block_sum_then_1d(double acc, double *part, Sc3 
 // inverse transform along x of two rows at once (the complex row X_a + i X_b,
 // each spectrum extended by its Hermitian symmetry; row a comes back as the
 // real part, row b as the imaginary part), z = s u, and r.z
-template <class F>
-__global__ void __launch_bounds__(256) k3s_inv_x(Dom3 d, SpecDims sd, const double2 *__restrict__ SP,
-                                                 const double *__restrict__ M, const double *__restrict__ R,
-                                                 double *__restrict__ Z, const double2 *__restrict__ TW,
-                                                 const int *gate, double *part, Sc3 *sc, F then)
+template <int LOGN, class F>
+__global__ void __launch_bounds__(XT, 2) k3s_inv_x(Dom3 d, SpecDims sd, const double2 *__restrict__ SP,
+                                                   const double *__restrict__ SM, const double *__restrict__ R,
+                                                   double *__restrict__ Z, const double2 *__restrict__ TW,
+                                                   const int *gate, double *part, Sc3 *sc, F then)
 {
-    extern __shared__ double2 sm[];
+    constexpr int N = 1 << LOGN, T = N / 8, G = XT / T, H = N / 2 + 1;
+    __shared__ double2 sm[G * (N + N / 8)];
     if (gate && *gate == 0) return;
-    double2 *w = sm, *a = sm + sd.N / 2 + (threadIdx.x / sd.nt_x) * sd.N;
-    fft_twiddles(w, TW, sd.N, 1.0);
-    const int g = threadIdx.x / sd.nt_x, t = threadIdx.x % sd.nt_x;
+    const int g = threadIdx.x / T, b = threadIdx.x % T;
+    double2 *a = sm + g * (N + N / 8);
     const long long rows = (long long)sd.K * sd.ny;
-    const long long ra = 2 * ((long long)blockIdx.x * sd.g_x + g), rb = ra + 1;
+    const long long ra = 2 * ((long long)blockIdx.x * G + g), rb = ra + 1;
     const bool la = ra < rows, lb = rb < rows;
-    const int ja = la ? (int)(ra % sd.ny) : 0, ka = la ? (int)(ra / sd.ny) : 0;
-    const int jb = lb ? (int)(rb % sd.ny) : 0, kb = lb ? (int)(rb / sd.ny) : 0;
-    for (int kx = t; kx < sd.N; kx += sd.nt_x) {
-        const bool lo = kx < sd.H;
-        const int c = lo ? kx : sd.N - kx;
-        const double sg = lo ? 1.0 : -1.0;
-        double2 xa = make_double2(0.0, 0.0), xb = make_double2(0.0, 0.0);
-        if (la) {
-            const double2 v = SP[ra * sd.H + c];
-            xa = make_double2(v.x, sg * v.y);
+    double2 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const int kx = b + T * k;
+        const bool lo = kx < H;
+        const int c = lo ? kx : N - kx;
+        double2 xa = la ? SP[ra * H + c] : make_double2(0.0, 0.0), xb = lb ? SP[rb * H + c] : make_double2(0.0, 0.0);
+        if (!lo) {
+            xa.y = -xa.y;
+            xb.y = -xb.y;
         }
-        if (lb) {
-            const double2 v = SP[rb * sd.H + c];
-            xb = make_double2(v.x, sg * v.y);
-        }
-        a[kx] = make_double2(xa.x - xb.y, xa.y + xb.x);
+        v[k] = make_double2(xa.x - xb.y, xa.y + xb.x);
     }
-    __syncthreads();
-    fft_group(a, w, sd.N, sd.logN, t, sd.nt_x);
+    auto sync = [] { if (T <= 32) __syncwarp(); else __syncthreads(); };
+    fft_regs<LOGN, true>(v, b, TW, [&](int i, double2 x) { a[i + (i >> 3)] = x; }, [&](int i) { return a[i + (i >> 3)]; }, sync);
+    const long long qa = la ? at(d, b, (int)(ra % sd.ny), (int)(ra / sd.ny)) : 0;
+    const long long qb = lb ? at(d, b, (int)(rb % sd.ny), (int)(rb / sd.ny)) : 0;
     double acc = 0.0;
-    for (int i = t; i < sd.N; i += sd.nt_x) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
         if (la) {
-            const long long q = at(d, i, ja, ka);
-            const double z = sqrt(M[q]) * a[i].x;
-            Z[q] = z;
-            acc += R[q] * z;
+            const double z = SM[qa + T * k] * v[k].x;
+            acc += R[qa + T * k] * z;
+            Z[qa + T * k] = z;
         }
         if (lb) {
-            const long long q = at(d, i, jb, kb);
-            const double z = sqrt(M[q]) * a[i].y;
-            Z[q] = z;
-            acc += R[q] * z;
+            const double z = SM[qb + T * k] * v[k].y;
+            acc += R[qb + T * k] * z;
+            Z[qb + T * k] = z;
         }
     }
     block_sum_then_1d(acc, part, sc, then);
@@ -785,10 +840,10 @@ struct GpuExec {
     }
     // spectral preconditioner: spectrum, tridiagonal tables, launch shapes
     double2 *spec = nullptr;
-    double *tri_cp = nullptr, *tri_im = nullptr;
+    double *tri_im = nullptr;
     SpecDims sd{};
     double spec_scale = 0.0;
-    double2 *tw_x = nullptr, *tw_z = nullptr;   // exp(-2 pi i q / n), q < n/2
+    double2 *tw_x = nullptr, *tw_z = nullptr;   // exp(-2 pi i q / n), q < n
     // z = s (-L)^-1 (s r) over the physical cells (the k3s_* kernels), then
     // r.z and the scalar step then(sc, r.z) in the last block
     // x transforms: one pair of rows per nt_x threads, g_x pairs per block
@@ -796,26 +851,54 @@ struct GpuExec {
     {
         return (((long long)sd.K * sd.ny + 1) / 2 + sd.g_x - 1) / sd.g_x;
     }
-    template <class F>
-    void spec_apply(const Dom3 &d, const double *R, const double *M, double *Z, const int *gate, F then)
+    template <int LOGN>
+    void launch_fwd_x(unsigned grid, const Dom3 &d, const double *R, const double *SM, const int *gate)
     {
-        const size_t smx = (size_t)(sd.N / 2 + sd.g_x * sd.N) * sizeof(double2);
-        const size_t smz = (size_t)(sd.K / 2 + sd.ch_z * sd.K) * sizeof(double2);
+        k3s_fwd_x<LOGN><<<grid, XT, 0, stream>>>(d, sd, R, SM, spec, tw_x, gate);
+        note();
+    }
+    template <int LOGN, class F>
+    void launch_inv_x(unsigned grid, const Dom3 &d, const double *R, const double *SM, double *Z, const int *gate, F then)
+    {
+        k3s_inv_x<LOGN><<<grid, XT, 0, stream>>>(d, sd, spec, SM, R, Z, tw_x, gate, part + (size_t)(NSLOT - 1) * pstride, sc, then);
+        note();
+    }
+    template <int LOGK>
+    void launch_z(bool inverse, const int *gate)
+    {
+        constexpr int T = (1 << LOGK) / 8;
+        const unsigned grid = (unsigned)(sd.ny * ((sd.H + sd.ch_z - 1) / sd.ch_z));
+        if (inverse) k3s_z<LOGK, true><<<grid, T * sd.ch_z, 0, stream>>>(sd, spec, tw_z, gate);
+        else k3s_z<LOGK, false><<<grid, T * sd.ch_z, 0, stream>>>(sd, spec, tw_z, gate);
+        note();
+    }
+    // f with the transform length 2^log as a compile-time constant (3 .. 10)
+    template <class F>
+    static void with_log(int log, F f)
+    {
+        switch (log) {
+        case 3: f(std::integral_constant<int, 3>()); break;
+        case 4: f(std::integral_constant<int, 4>()); break;
+        case 5: f(std::integral_constant<int, 5>()); break;
+        case 6: f(std::integral_constant<int, 6>()); break;
+        case 7: f(std::integral_constant<int, 7>()); break;
+        case 8: f(std::integral_constant<int, 8>()); break;
+        case 9: f(std::integral_constant<int, 9>()); break;
+        default: f(std::integral_constant<int, 10>()); break;
+        }
+    }
+    template <class F>
+    void spec_apply(const Dom3 &d, const double *R, const double *SM, double *Z, const int *gate, F then)
+    {
         const unsigned gx = (unsigned)spec_xblocks(sd);
-        const unsigned gz = (unsigned)(sd.ny * ((sd.H + sd.ch_z - 1) / sd.ch_z));
         // one thread per system, a few thousand systems: blocks of 32 spread them over every SM
         const unsigned gt = (unsigned)(((long long)sd.K * sd.H + 31) / 32);
-        k3s_fwd_x<<<gx, 256, smx, stream>>>(d, sd, R, M, spec, tw_x, gate);
+        with_log(sd.logN, [&](auto L) { launch_fwd_x<decltype(L)::value>(gx, d, R, SM, gate); });
+        with_log(sd.logK, [&](auto L) { launch_z<decltype(L)::value>(false, gate); });
+        k3s_tri<<<gt, 32, 0, stream>>>(sd, spec, tri_im, spec_scale, gate);
         note();
-        k3s_z<<<gz, 256, smz, stream>>>(sd, spec, tw_z, -1.0, gate);
-        note();
-        k3s_tri<<<gt, 32, 0, stream>>>(sd, spec, tri_cp, tri_im, spec_scale, gate);
-        note();
-        k3s_z<<<gz, 256, smz, stream>>>(sd, spec, tw_z, 1.0, gate);
-        note();
-        k3s_inv_x<<<gx, 256, smx, stream>>>(d, sd, spec, M, R, Z, tw_x, gate, part + (size_t)(NSLOT - 1) * pstride, sc,
-                                             then);
-        note();
+        with_log(sd.logK, [&](auto L) { launch_z<decltype(L)::value>(true, gate); });
+        with_log(sd.logN, [&](auto L) { launch_inv_x<decltype(L)::value>(gx, d, R, SM, Z, gate, then); });
     }
     void p_dir_z(const Dom3 &d, const double *Z, double *DD, const int *gate)
     {
@@ -895,7 +978,6 @@ int destroy(Handle *h)
     cudaFree(x.sc);
     cudaFree(x.part);
     cudaFree(x.spec);
-    cudaFree(x.tri_cp);
     cudaFree(x.tri_im);
     cudaFree(x.tw_x);
     cudaFree(x.tw_z);
@@ -923,16 +1005,12 @@ static int spec_setup(GpuExec &x, const Dom3 &d, const pvof_grid_desc *g)
     while ((1 << sd.logN) < sd.N) sd.logN++;
     sd.logK = 0;
     while ((1 << sd.logK) < sd.K) sd.logK++;
-    sd.nt_x = std::min(256, sd.N / 2);
-    sd.g_x = 256 / sd.nt_x;
-    int ch = (int)((48 * 1024 / sizeof(double2) - sd.K / 2) / sd.K);
-    sd.ch_z = 1;
-    while (sd.ch_z * 2 <= std::min(ch, 16)) sd.ch_z *= 2;
-    sd.nt_z = 256 / sd.ch_z;
+    sd.g_x = XT / (sd.N / 8);
+    sd.ch_z = std::min(32, 256 / (sd.K / 8));
     const double idy2 = d.idy2;
     x.spec_scale = (1.0 / idy2) / ((double)sd.N * (double)sd.K);
     const size_t n = (size_t)sd.K * sd.ny * sd.H;
-    std::vector<double> cp(n), im(n);
+    std::vector<double> im(n);
     const double pi = 3.14159265358979323846;
     for (int kz = 0; kz < sd.K; kz++)
         for (int kx = 0; kx < sd.H; kx++) {
@@ -944,24 +1022,22 @@ static int spec_setup(GpuExec &x, const Dom3 &d, const pvof_grid_desc *g)
                 const double m = b + cprev;
                 const size_t q = ((size_t)kz * sd.ny + j) * sd.H + kx;
                 im[q] = 1.0 / m;
-                cp[q] = -1.0 / m;
-                cprev = cp[q];
+                cprev = -im[q];
             }
         }
     (void)g;
-    std::vector<double2> twx((size_t)sd.N / 2), twz((size_t)sd.K / 2);
-    for (int q = 0; q < sd.N / 2; q++) twx[q] = make_double2(std::cos(2.0 * pi * q / sd.N), -std::sin(2.0 * pi * q / sd.N));
-    for (int q = 0; q < sd.K / 2; q++) twz[q] = make_double2(std::cos(2.0 * pi * q / sd.K), -std::sin(2.0 * pi * q / sd.K));
+    std::vector<double2> twx((size_t)sd.N), twz((size_t)sd.K);
+    for (int q = 0; q < sd.N; q++) twx[q] = make_double2(std::cos(2.0 * pi * q / sd.N), -std::sin(2.0 * pi * q / sd.N));
+    for (int q = 0; q < sd.K; q++) twz[q] = make_double2(std::cos(2.0 * pi * q / sd.K), -std::sin(2.0 * pi * q / sd.K));
     if (cudaMalloc(&x.tw_x, twx.size() * sizeof(double2)) != cudaSuccess ||
         cudaMalloc(&x.tw_z, twz.size() * sizeof(double2)) != cudaSuccess ||
         cudaMemcpy(x.tw_x, twx.data(), twx.size() * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(x.tw_z, twz.data(), twz.size() * sizeof(double2), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(PVOF_ENOMEM, "twiddle tables");
-    if (cudaMalloc(&x.spec, n * sizeof(double2)) != cudaSuccess || cudaMalloc(&x.tri_cp, n * sizeof(double)) != cudaSuccess ||
+    if (cudaMalloc(&x.spec, n * sizeof(double2)) != cudaSuccess ||
         cudaMalloc(&x.tri_im, n * sizeof(double)) != cudaSuccess)
         return fail(PVOF_ENOMEM, "device memory for the spectral preconditioner");
-    if (cudaMemcpy(x.tri_cp, cp.data(), n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(x.tri_im, im.data(), n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpy(x.tri_im, im.data(), n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
         return fail(PVOF_ECUDA, "spectral tables upload");
     return PVOF_OK;
 }

@@ -371,7 +371,8 @@ enum F3 {
     F3_U_EXO, F3_U_VXO, F3_U_RHS, F3_V_EXO, F3_V_VXO, F3_V_RHS, F3_W_EXO, F3_W_VXO, F3_W_RHS,
     F3_VR, F3_VD, F3_VAD, F3_VDIAG,
     F3_FSO_X, F3_FSO_Y, F3_FSO_Z, F3_FSN_X, F3_FSN_Y, F3_FSN_Z,
-    F3_PCX, F3_PCY, F3_PCZ, F3_PZ,
+    F3_PCX, F3_PCY, F3_PCZ, F3_PZ, F3_PSM,
+    F3_VFT, F3_VMU, F3_VMA, F3_VMB,
     F3_COUNT
 };
 
@@ -546,105 +547,108 @@ __host__ __device__ __forceinline__ MomTerms mom_terms(const Dom3 &d, const Phas
     return t;
 }
 
-// vel_jacobi_diag and one row of matVec (msolve_cg.c:103-493, VOF branch)
-// of component C at (i,j,k); x is read through the ghost update KX
+// The coefficients of vel_jacobi_diag and matVec (msolve_cg.c:98-493, VOF
+// branch) of component C at a face, stored once per solve: the time term ft, the
+// viscosity of the cell above the face, and the two corner viscosities on its
+// upper sides, ma (in the first direction other than C) and mb (in the second).  The lower corner of a face is the upper
+// corner of the face below it in that direction: the same expression with the
+// same operands, so a face reads it there (the ranges start with one more
+// layer, see vel_weights_range).
 template <int C>
-__host__ __device__ __forceinline__ double vel_diag(const Dom3 &d, const Phase &ph, double iRe, double alpha_k,
-                                                    double dt, const double *CL, int i, int j, int k)
+__host__ __device__ __forceinline__ void vel_weights(const Dom3 &d, const Phase &ph, double alpha_k, double dt, const double *CL,
+                                                     double *FT, double *MU, double *MA, double *MB, int i, int j, int k)
 {
     auto mu = [&](int a, int b, int e) { return ph.mu(rd<K_SCALAR>(d, CL, a, b, e)); };
     auto rho = [&](int a, int b, int e) { return ph.rho(rd<K_SCALAR>(d, CL, a, b, e)); };
+    const long long q = at(d, i, j, k);
     const double rho_face = 0.5 * (rho(i, j, k) + rho(C == 0 ? i - 1 : i, C == 1 ? j - 1 : j, C == 2 ? k - 1 : k));
-    const double d_time = rho_face / (alpha_k * dt);
-    double dx, dy, dz, dax = 0.0;
+    FT[q] = rho_face / (alpha_k * dt);
+    MU[q] = mu(i, j, k);
     if (C == 0) {
-        const double mu_xp = mu(i, j, k), mu_xm = mu(i - 1, j, k);
-        const double mu_yp = harm(avg2(mu(i - 1, j + 1, k), mu(i, j + 1, k)), avg2(mu(i - 1, j, k), mu(i, j, k)));
-        const double mu_ym = harm(avg2(mu(i - 1, j, k), mu(i, j, k)), avg2(mu(i - 1, j - 1, k), mu(i, j - 1, k)));
-        const double mu_zp = harm(avg2(mu(i - 1, j, k + 1), mu(i, j, k + 1)), avg2(mu(i - 1, j, k), mu(i, j, k)));
-        const double mu_zm = harm(avg2(mu(i - 1, j, k), mu(i, j, k)), avg2(mu(i - 1, j, k - 1), mu(i, j, k - 1)));
-        dx = iRe * ((mu_xp * d.idx_u[i] + mu_xm * d.idx_u[i - 1]) * d.idx_c[i - 1]);
-        dy = iRe * (mu_yp * d.idy_c[j] + mu_ym * d.idy_c[j - 1]) * d.idy_v[j];
-        dz = iRe * (mu_zp * d.idz_c[k] + mu_zm * d.idz_c[k - 1]) * d.idz_w[k];
+        MA[q] = harm(avg2(mu(i - 1, j + 1, k), mu(i, j + 1, k)), avg2(mu(i - 1, j, k), mu(i, j, k)));
+        MB[q] = harm(avg2(mu(i - 1, j, k + 1), mu(i, j, k + 1)), avg2(mu(i - 1, j, k), mu(i, j, k)));
     } else if (C == 1) {
-        const double mu_yp = mu(i, j, k), mu_ym = mu(i, j - 1, k);
-        const double mu_xp = harm(avg2(mu(i + 1, j - 1, k), mu(i + 1, j, k)), avg2(mu(i, j - 1, k), mu(i, j, k)));
-        const double mu_xm = harm(avg2(mu(i, j - 1, k), mu(i, j, k)), avg2(mu(i - 1, j - 1, k), mu(i - 1, j, k)));
-        const double mu_zp = harm(avg2(mu(i, j - 1, k + 1), mu(i, j, k + 1)), avg2(mu(i, j - 1, k), mu(i, j, k)));
-        const double mu_zm = harm(avg2(mu(i, j - 1, k), mu(i, j, k)), avg2(mu(i, j - 1, k - 1), mu(i, j, k - 1)));
-        dx = iRe * ((mu_xp * d.idx_c[i] + mu_xm * d.idx_c[i - 1]) * d.idx_u[i]);
-        dy = iRe * (mu_yp * d.idy_v[j] + mu_ym * d.idy_v[j - 1]) * d.idy_c[j - 1];
-        dz = iRe * (mu_zp * d.idz_c[k] + mu_zm * d.idz_c[k - 1]) * d.idz_w[k];
+        MA[q] = harm(avg2(mu(i + 1, j - 1, k), mu(i + 1, j, k)), avg2(mu(i, j - 1, k), mu(i, j, k)));
+        MB[q] = harm(avg2(mu(i, j - 1, k + 1), mu(i, j, k + 1)), avg2(mu(i, j - 1, k), mu(i, j, k)));
     } else {
-        const double mu_zp = mu(i, j, k), mu_zm = mu(i, j, k - 1);
-        const double mu_xp = harm(avg2(mu(i + 1, j, k - 1), mu(i + 1, j, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
-        const double mu_xm = harm(avg2(mu(i, j, k - 1), mu(i, j, k)), avg2(mu(i - 1, j, k - 1), mu(i - 1, j, k)));
-        const double mu_yp = harm(avg2(mu(i, j + 1, k - 1), mu(i, j + 1, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
-        const double mu_ym = harm(avg2(mu(i, j, k - 1), mu(i, j, k)), avg2(mu(i, j - 1, k - 1), mu(i, j - 1, k)));
-        dx = iRe * (mu_xp * d.idx_c[i] + mu_xm * d.idx_c[i - 1]) * d.idx_u[i];
-        dy = iRe * (mu_yp * d.idy_c[j] + mu_ym * d.idy_c[j - 1]) * d.idy_v[j];
-        dz = iRe * (mu_zp * d.idz_w[k] + mu_zm * d.idz_w[k - 1]) * d.idz_c[k - 1];
+        MA[q] = harm(avg2(mu(i + 1, j, k - 1), mu(i + 1, j, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
+        MB[q] = harm(avg2(mu(i, j + 1, k - 1), mu(i, j + 1, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
     }
-    return d_time + dx + dy + dz + dax;
+}
+// the faces of component C and the layers just below them that they read
+inline Range vel_weights_range(const Range &r, int comp)
+{
+    return Range{r.i0 - 1, r.i1, r.j0 - 1, r.j1, r.k0 - 1, r.k1};
 }
 
-template <int C, int KX>
-__host__ __device__ __forceinline__ double vel_op(const Dom3 &d, const Phase &ph, double iRe, double alpha_k, double dt,
-                                                  const double *CL, const double *X, int i, int j, int k)
+// vel_jacobi_diag (msolve_cg.c:98-249) from vel_weights' fields
+template <int C>
+__host__ __device__ __forceinline__ double vel_diag_w(const Dom3 &d, double iRe, const double *FT, const double *MU,
+                                                      const double *MA, const double *MB, int i, int j, int k)
 {
-    auto mu = [&](int a, int b, int e) { return ph.mu(rd<K_SCALAR>(d, CL, a, b, e)); };
-    auto rho = [&](int a, int b, int e) { return ph.rho(rd<K_SCALAR>(d, CL, a, b, e)); };
+    const long long q = at(d, i, j, k), di = 1, dj = d.P, dk = d.S;
+    double dx, dy, dz, dax = 0.0;
+    if (C == 0) {
+        dx = iRe * ((MU[q] * d.idx_u[i] + MU[q - di] * d.idx_u[i - 1]) * d.idx_c[i - 1]);
+        dy = iRe * (MA[q] * d.idy_c[j] + MA[q - dj] * d.idy_c[j - 1]) * d.idy_v[j];
+        dz = iRe * (MB[q] * d.idz_c[k] + MB[q - dk] * d.idz_c[k - 1]) * d.idz_w[k];
+    } else if (C == 1) {
+        dx = iRe * ((MA[q] * d.idx_c[i] + MA[q - di] * d.idx_c[i - 1]) * d.idx_u[i]);
+        dy = iRe * (MU[q] * d.idy_v[j] + MU[q - dj] * d.idy_v[j - 1]) * d.idy_c[j - 1];
+        dz = iRe * (MB[q] * d.idz_c[k] + MB[q - dk] * d.idz_c[k - 1]) * d.idz_w[k];
+    } else {
+        dx = iRe * (MA[q] * d.idx_c[i] + MA[q - di] * d.idx_c[i - 1]) * d.idx_u[i];
+        dy = iRe * (MB[q] * d.idy_c[j] + MB[q - dj] * d.idy_c[j - 1]) * d.idy_v[j];
+        dz = iRe * (MU[q] * d.idz_w[k] + MU[q - dk] * d.idz_w[k - 1]) * d.idz_c[k - 1];
+    }
+    return FT[q] + dx + dy + dz + dax;
+}
+
+// one row of matVec (msolve_cg.c:255-493) from vel_weights' fields; x is read
+// through the ghost update KX.  No division and one viscosity per neighbour
+// where evaluating them from C_L at every application took ten divisions and
+// up to 18 phase cells: 120x97x104 78 -> 33 us an application.
+template <int C, int KX>
+__host__ __device__ __forceinline__ double vel_op_w(const Dom3 &d, double iRe, const double *FT, const double *MU, const double *MA,
+                                                    const double *MB, const double *X, int i, int j, int k)
+{
     auto x = [&](int a, int b, int e) { return rd<KX>(d, X, a, b, e); };
-    const double rho_face = 0.5 * (rho(i, j, k) + rho(C == 0 ? i - 1 : i, C == 1 ? j - 1 : j, C == 2 ? k - 1 : k));
-    const double factor_time = rho_face / (alpha_k * dt);
+    const long long q = at(d, i, j, k), di = 1, dj = d.P, dk = d.S;
     const double xc = x(i, j, k);
-    const double Ax = factor_time * xc;
+    const double Ax = FT[q] * xc;
+    const double xp = x(i + 1, j, k), xm = x(i - 1, j, k), yp = x(i, j + 1, k), ym = x(i, j - 1, k), zp = x(i, j, k + 1),
+                 zm = x(i, j, k - 1);
     double op = 0.0;
     if (C == 0) {
-        const double mu_xp = mu(i, j, k), mu_xm = mu(i - 1, j, k);
-        const double mu_yp = harm(avg2(mu(i - 1, j + 1, k), mu(i, j + 1, k)), avg2(mu(i - 1, j, k), mu(i, j, k)));
-        const double mu_ym = harm(avg2(mu(i - 1, j, k), mu(i, j, k)), avg2(mu(i - 1, j - 1, k), mu(i, j - 1, k)));
-        const double mu_zp = harm(avg2(mu(i - 1, j, k + 1), mu(i, j, k + 1)), avg2(mu(i - 1, j, k), mu(i, j, k)));
-        const double mu_zm = harm(avg2(mu(i - 1, j, k), mu(i, j, k)), avg2(mu(i - 1, j, k - 1), mu(i, j, k - 1)));
-        const double fxp = mu_xp * (x(i + 1, j, k) - xc) * d.idx_u[i];
-        const double fxm = mu_xm * (xc - x(i - 1, j, k)) * d.idx_u[i - 1];
-        const double fyp = mu_yp * (x(i, j + 1, k) - xc) * d.idy_c[j];
-        const double fym = mu_ym * (xc - x(i, j - 1, k)) * d.idy_c[j - 1];
+        const double fxp = MU[q] * (xp - xc) * d.idx_u[i];
+        const double fxm = MU[q - di] * (xc - xm) * d.idx_u[i - 1];
+        const double fyp = MA[q] * (yp - xc) * d.idy_c[j];
+        const double fym = MA[q - dj] * (xc - ym) * d.idy_c[j - 1];
         op += iRe * ((fxp - fxm) * d.idx_c[i - 1]);
         op += iRe * (fyp - fym) * d.idy_v[j];
-        const double fzp = mu_zp * (x(i, j, k + 1) - xc) * d.idz_c[k];
-        const double fzm = mu_zm * (xc - x(i, j, k - 1)) * d.idz_c[k - 1];
+        const double fzp = MB[q] * (zp - xc) * d.idz_c[k];
+        const double fzm = MB[q - dk] * (xc - zm) * d.idz_c[k - 1];
         op += iRe * (fzp - fzm) * d.idz_w[k];
         op += 0.0;
     } else if (C == 1) {
-        const double mu_yp = mu(i, j, k), mu_ym = mu(i, j - 1, k);
-        const double mu_xp = harm(avg2(mu(i + 1, j - 1, k), mu(i + 1, j, k)), avg2(mu(i, j - 1, k), mu(i, j, k)));
-        const double mu_xm = harm(avg2(mu(i, j - 1, k), mu(i, j, k)), avg2(mu(i - 1, j - 1, k), mu(i - 1, j, k)));
-        const double mu_zp = harm(avg2(mu(i, j - 1, k + 1), mu(i, j, k + 1)), avg2(mu(i, j - 1, k), mu(i, j, k)));
-        const double mu_zm = harm(avg2(mu(i, j - 1, k), mu(i, j, k)), avg2(mu(i, j - 1, k - 1), mu(i, j, k - 1)));
-        const double fxp = mu_xp * (x(i + 1, j, k) - xc) * d.idx_c[i];
-        const double fxm = mu_xm * (xc - x(i - 1, j, k)) * d.idx_c[i - 1];
-        const double fyp = mu_yp * (x(i, j + 1, k) - xc) * d.idy_v[j];
-        const double fym = mu_ym * (xc - x(i, j - 1, k)) * d.idy_v[j - 1];
+        const double fxp = MA[q] * (xp - xc) * d.idx_c[i];
+        const double fxm = MA[q - di] * (xc - xm) * d.idx_c[i - 1];
+        const double fyp = MU[q] * (yp - xc) * d.idy_v[j];
+        const double fym = MU[q - dj] * (xc - ym) * d.idy_v[j - 1];
         op += iRe * ((fxp - fxm) * d.idx_u[i]);
         op += iRe * (fyp - fym) * d.idy_c[j - 1];
-        const double fzp = mu_zp * (x(i, j, k + 1) - xc) * d.idz_c[k];
-        const double fzm = mu_zm * (xc - x(i, j, k - 1)) * d.idz_c[k - 1];
+        const double fzp = MB[q] * (zp - xc) * d.idz_c[k];
+        const double fzm = MB[q - dk] * (xc - zm) * d.idz_c[k - 1];
         op += iRe * (fzp - fzm) * d.idz_w[k];
     } else {
-        const double mu_zp = mu(i, j, k), mu_zm = mu(i, j, k - 1);
-        const double mu_xp = harm(avg2(mu(i + 1, j, k - 1), mu(i + 1, j, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
-        const double mu_xm = harm(avg2(mu(i, j, k - 1), mu(i, j, k)), avg2(mu(i - 1, j, k - 1), mu(i - 1, j, k)));
-        const double mu_yp = harm(avg2(mu(i, j + 1, k - 1), mu(i, j + 1, k)), avg2(mu(i, j, k - 1), mu(i, j, k)));
-        const double mu_ym = harm(avg2(mu(i, j, k - 1), mu(i, j, k)), avg2(mu(i, j - 1, k - 1), mu(i, j - 1, k)));
-        const double fxp = mu_xp * (x(i + 1, j, k) - xc) * d.idx_c[i];
-        const double fxm = mu_xm * (xc - x(i - 1, j, k)) * d.idx_c[i - 1];
-        const double fyp = mu_yp * (x(i, j + 1, k) - xc) * d.idy_c[j];
-        const double fym = mu_ym * (xc - x(i, j - 1, k)) * d.idy_c[j - 1];
+        const double fxp = MA[q] * (xp - xc) * d.idx_c[i];
+        const double fxm = MA[q - di] * (xc - xm) * d.idx_c[i - 1];
+        const double fyp = MB[q] * (yp - xc) * d.idy_c[j];
+        const double fym = MB[q - dj] * (xc - ym) * d.idy_c[j - 1];
         op += iRe * (fxp - fxm) * d.idx_u[i];
         op += iRe * (fyp - fym) * d.idy_v[j];
-        const double fzp = mu_zp * (x(i, j, k + 1) - xc) * d.idz_w[k];
-        const double fzm = mu_zm * (xc - x(i, j, k - 1)) * d.idz_w[k - 1];
+        const double fzp = MU[q] * (zp - xc) * d.idz_w[k];
+        const double fzm = MU[q - dk] * (xc - zm) * d.idz_w[k - 1];
         op += iRe * (fzp - fzm) * d.idz_c[k - 1];
     }
     return Ax - op;
@@ -1049,6 +1053,7 @@ struct Box3 {
         Sc3 *sc = x.sc;
         const double *CL = f[F3_CL], *RHS = f[F3_U_RHS + 3 * C];
         double *DATA = f[F3_U + C], *R = f[F3_VR], *AD = f[F3_VAD], *DG = f[F3_VDIAG], *DD = vd[C];
+        double *FT = f[F3_VFT], *MU = f[F3_VMU], *MA = f[F3_VMA], *MB = f[F3_VMB];
         const double iRe = 1.0 / p.Re, alpha_k = bet(stage), dt = this->dt;
         const double EPS = p.velocity_cg_unregularized ? 0.0 : 1e-14;
         const int NX = d.NX, NY = d.NY, NZ = d.NZ;
@@ -1057,9 +1062,12 @@ struct Box3 {
         const double tol = p.CG_ETOL;
         const int maxit = p.CG_MAXIT;
         const Range fr = face_range(d, C);
+        x.cells(vel_weights_range(fr, C), nullptr, [=] __host__ __device__(int i, int j, int k) {
+            vel_weights<C>(d, ph, alpha_k, dt, CL, FT, MU, MA, MB, i, j, k);
+        });
         x.template reduce<1>(fr, nullptr, 0, [=] __host__ __device__(int i, int j, int k) {
-            const double dg = vel_diag<C>(d, ph, iRe, alpha_k, dt, CL, i, j, k);
-            const double ad = vel_op<C, KN>(d, ph, iRe, alpha_k, dt, CL, DATA, i, j, k);
+            const double dg = vel_diag_w<C>(d, iRe, FT, MU, MA, MB, i, j, k);
+            const double ad = vel_op_w<C, KN>(d, iRe, FT, MU, MA, MB, DATA, i, j, k);
             const long long q = at(d, i, j, k);
             DG[q] = dg;
             const double r = RHS[q] - ad;
@@ -1082,7 +1090,7 @@ struct Box3 {
         for (int it = 0; it < maxit; it += CHUNK) {
             for (int q = 0; q < CHUNK && it + q < maxit; q++) {
                 x.template reduce<1>(fr, gate, 0, [=] __host__ __device__(int i, int j, int k) {
-                    const double ad = vel_op<C, KC>(d, ph, iRe, alpha_k, dt, CL, DD, i, j, k);
+                    const double ad = vel_op_w<C, KC>(d, iRe, FT, MU, MA, MB, DD, i, j, k);
                     const long long q = at(d, i, j, k);
                     AD[q] = ad;
                     return Vec<1>{{DD[q] * ad}};
@@ -1159,7 +1167,7 @@ struct Box3 {
         const Dom3 d = this->d;
         Sc3 *sc = x.sc;
         const double *B = f[F3_PRHS], *M = f[F3_PM], *CX = f[F3_PCX], *CY = f[F3_PCY], *CZ = f[F3_PCZ];
-        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD], *Z = f[F3_PZ];
+        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD], *Z = f[F3_PZ], *SM = f[F3_PSM];
         const double tol = p.P_CG_ETOL;
         const int maxit = p.P_CG_MAXIT;
         const Range cr = cells_range(d);
@@ -1167,10 +1175,11 @@ struct Box3 {
             const long long q = at(d, i, j, k);
             const double r = B[q] - p_apply_st(d, CX, CY, CZ, PHI, i, j, k);
             R[q] = r;
+            SM[q] = sqrt(M[q]);
             return Vec<1>{{r * (r * M[q])}};
         });
         // z = P r and gamma = r.z, then d = z
-        x.spec_apply(d, R, M, Z, nullptr, [=] __host__ __device__(Sc3 * s, double rz) {
+        x.spec_apply(d, R, SM, Z, nullptr, [=] __host__ __device__(Sc3 * s, double rz) {
             s->p_gamma = rz;
             s->p_beta = 0.0;
         });
@@ -1196,7 +1205,7 @@ struct Box3 {
                     if (sqrt(rMr) < s->p_tol) s->p_active = 0;
                 });
                 // z = P r, r.z and the direction's coefficient, then d = z + beta d
-                x.spec_apply(d, R, M, Z, gate, [=] __host__ __device__(Sc3 * s, double g) {
+                x.spec_apply(d, R, SM, Z, gate, [=] __host__ __device__(Sc3 * s, double g) {
                     s->p_beta = g / (s->p_gamma + 1e-300);
                     s->p_gamma = g;
                     if (s->p_iter >= s->p_maxit) s->p_active = 0;
