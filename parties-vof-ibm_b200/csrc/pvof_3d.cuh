@@ -372,7 +372,7 @@ enum F3 {
     F3_VR, F3_VD, F3_VAD, F3_VDIAG,
     F3_FSO_X, F3_FSO_Y, F3_FSO_Z, F3_FSN_X, F3_FSN_Y, F3_FSN_Z,
     F3_PCX, F3_PCY, F3_PCZ, F3_PZ, F3_PSM,
-    F3_VFT, F3_VMU, F3_VMA, F3_VMB,
+    F3_VFT, F3_VMU, F3_VMA, F3_VMB, F3_VZ, F3_VD2, F3_VZ_V, F3_VD2_V, F3_PD2,
     F3_COUNT
 };
 
@@ -604,15 +604,14 @@ __host__ __device__ __forceinline__ double vel_diag_w(const Dom3 &d, double iRe,
     return FT[q] + dx + dy + dz + dax;
 }
 
-// one row of matVec (msolve_cg.c:255-493) from vel_weights' fields; x is read
-// through the ghost update KX.  No division and one viscosity per neighbour
+// one row of matVec (msolve_cg.c:255-493) from vel_weights' fields, x(i,j,k) the
+// vector after its ghost update.  No division and one viscosity per neighbour
 // where evaluating them from C_L at every application took ten divisions and
 // up to 18 phase cells: 120x97x104 78 -> 33 us an application.
-template <int C, int KX>
+template <int C, class Get>
 __host__ __device__ __forceinline__ double vel_op_w(const Dom3 &d, double iRe, const double *FT, const double *MU, const double *MA,
-                                                    const double *MB, const double *X, int i, int j, int k)
+                                                    const double *MB, int i, int j, int k, Get x)
 {
-    auto x = [&](int a, int b, int e) { return rd<KX>(d, X, a, b, e); };
     const long long q = at(d, i, j, k), di = 1, dj = d.P, dk = d.S;
     const double xc = x(i, j, k);
     const double Ax = FT[q] * xc;
@@ -760,7 +759,11 @@ struct Box3 {
     int stage = 0;
     double dt = 0.0, time = 0.0, clamp_total = 0.0;
     bool initialized = false;
-    static constexpr int CHUNK = 8;   // CG iterations issued between two reads of the device flag
+    // CG iterations issued between two reads of the device flag: 8, then twice as
+    // many each time up to 32 (a long solve waits for the flag less often, a short
+    // one issues few gated launches past its end)
+    static constexpr int CHUNK = 8, CHUNK_MAX = 32;
+    static int next_chunk(int c) { return c < CHUNK_MAX ? 2 * c : c; }
     // solver counters (PVOF_SOLVER_BIHARMONIC, _VELOCITY, _PRESSURE): solves,
     // iterations, cell-iterations since the context was created
     long long sol_launches[3] = {}, sol_iters[3] = {}, sol_cell_iters[3] = {};
@@ -1042,7 +1045,11 @@ struct Box3 {
         });
     }
 
-    // Velocity_solve_cg (msolve_cg.c:525-722) of component C
+    // Velocity_solve_cg (msolve_cg.c:525-722) of component C.  Two passes per
+    // iteration: the executor's v_dir_op (x += alpha d of the iteration before,
+    // d = z + beta d on the fly at the face and its neighbours, A d and d.Ad) and
+    // v_resid (r -= alpha Ad, z = M^-1 r and the sums); the directions alternate
+    // between two fields by the parity of the iteration.
     template <int C>
     void velocity_solve()
     {
@@ -1052,8 +1059,11 @@ struct Box3 {
         const Phase ph = this->ph;
         Sc3 *sc = x.sc;
         const double *CL = f[F3_CL], *RHS = f[F3_U_RHS + 3 * C];
-        double *DATA = f[F3_U + C], *R = f[F3_VR], *AD = f[F3_VAD], *DG = f[F3_VDIAG], *DD = vd[C];
+        double *DATA = f[F3_U + C], *R = f[F3_VR], *AD = f[F3_VAD], *DG = f[F3_VDIAG];
         double *FT = f[F3_VFT], *MU = f[F3_VMU], *MA = f[F3_VMA], *MB = f[F3_VMB];
+        // the direction's wall faces of v read as stored (zero): fields that no
+        // other component writes
+        double *D0 = vd[C], *D1 = f[C == 1 ? F3_VD2_V : F3_VD2], *Z = f[C == 1 ? F3_VZ_V : F3_VZ];
         const double iRe = 1.0 / p.Re, alpha_k = bet(stage), dt = this->dt;
         const double EPS = p.velocity_cg_unregularized ? 0.0 : 1e-14;
         const int NX = d.NX, NY = d.NY, NZ = d.NZ;
@@ -1067,48 +1077,37 @@ struct Box3 {
         });
         x.template reduce<1>(fr, nullptr, 0, [=] __host__ __device__(int i, int j, int k) {
             const double dg = vel_diag_w<C>(d, iRe, FT, MU, MA, MB, i, j, k);
-            const double ad = vel_op_w<C, KN>(d, iRe, FT, MU, MA, MB, DATA, i, j, k);
+            const double ad = vel_op_w<C>(d, iRe, FT, MU, MA, MB, i, j, k,
+                                          [&](int a, int b, int e) { return rd<KN>(d, DATA, a, b, e); });
             const long long q = at(d, i, j, k);
             DG[q] = dg;
             const double r = RHS[q] - ad;
             R[q] = r;
-            const double dd = r / (dg + EPS);
-            DD[q] = dd;
-            return Vec<1>{{r * dd}};
+            const double z = r / (dg + EPS);
+            Z[q] = z;
+            return Vec<1>{{r * z}};
         });
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->v_rz = s->sum[0][0];
             s->v_iter = 0;
             s->v_maxit = maxit;
             s->v_rms = 0.0;
+            s->v_alpha = 0.0;
+            s->v_beta = 0.0;
             s->v_eps = EPS;
             s->v_in_tot = in_tot;
             s->v_tol = tol;
             s->v_active = maxit > 0 ? 1 : 0;
         });
         const int *gate = &sc->v_active;
-        for (int it = 0; it < maxit; it += CHUNK) {
-            for (int q = 0; q < CHUNK && it + q < maxit; q++) {
-                x.template reduce<1>(fr, gate, 0, [=] __host__ __device__(int i, int j, int k) {
-                    const double ad = vel_op_w<C, KC>(d, iRe, FT, MU, MA, MB, DD, i, j, k);
-                    const long long q = at(d, i, j, k);
-                    AD[q] = ad;
-                    return Vec<1>{{DD[q] * ad}};
-                });
-                x.scalar(gate, [=] __host__ __device__(Sc3 * s) {
+        for (int it = 0, chunk = CHUNK; it < maxit; it += chunk, chunk = next_chunk(chunk)) {
+            for (int q = 0; q < chunk && it + q < maxit; q++) {
+                x.template v_dir_op<C, KC>(d, fr, iRe, FT, MU, MA, MB, Z, D0, D1, DATA, AD, gate,
+                                           [=] __host__ __device__(Sc3 * s, double dAd) {
+                                               s->v_alpha = s->v_rz / (dAd + s->v_eps);
+                                           });
+                x.v_resid(d, fr, R, AD, DG, Z, gate, [=] __host__ __device__(Sc3 * s, double rz_new, double rr) {
                     s->v_iter++;
-                    s->v_alpha = s->v_rz / (s->sum[0][0] + s->v_eps);
-                });
-                x.template reduce<2>(fr, gate, 0, [=] __host__ __device__(int i, int j, int k) {
-                    const double alpha = sc->v_alpha, eps = sc->v_eps;
-                    const long long q = at(d, i, j, k);
-                    DATA[q] += alpha * DD[q];
-                    const double r = R[q] - alpha * AD[q];
-                    R[q] = r;
-                    return Vec<2>{{r * r / (DG[q] + eps), r * r}};
-                });
-                x.scalar(gate, [=] __host__ __device__(Sc3 * s) {
-                    const double rz_new = s->sum[0][0], rr = s->sum[0][1];
                     s->v_rms = sqrt(s->v_in_tot * rr);
                     if (s->v_rms < s->v_tol) {
                         s->v_active = 0;
@@ -1118,13 +1117,14 @@ struct Box3 {
                         if (s->v_iter >= s->v_maxit) s->v_active = 0;
                     }
                 });
-                x.cells(fr, gate, [=] __host__ __device__(int i, int j, int k) {
-                    const long long q = at(d, i, j, k);
-                    DD[q] = R[q] / (DG[q] + sc->v_eps) + sc->v_beta * DD[q];
-                });
             }
             if (!x.read_int(gate)) break;
         }
+        // the last iteration's update
+        x.cells(fr, &sc->v_iter, [=] __host__ __device__(int i, int j, int k) {
+            const long long q = at(d, i, j, k);
+            DATA[q] += sc->v_alpha * ((sc->v_iter & 1) ? D1 : D0)[q];
+        });
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->v_iters_out[C] = s->v_iter;
             s->v_rms_out[C] = s->v_rms;
@@ -1167,7 +1167,7 @@ struct Box3 {
         const Dom3 d = this->d;
         Sc3 *sc = x.sc;
         const double *B = f[F3_PRHS], *M = f[F3_PM], *CX = f[F3_PCX], *CY = f[F3_PCY], *CZ = f[F3_PCZ];
-        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD], *Z = f[F3_PZ], *SM = f[F3_PSM];
+        double *PHI = f[F3_DP], *R = f[F3_PR], *D0 = f[F3_PD], *D1 = f[F3_PD2], *AD = f[F3_PAD], *Z = f[F3_PZ], *SM = f[F3_PSM];
         const double tol = p.P_CG_ETOL;
         const int maxit = p.P_CG_MAXIT;
         const Range cr = cells_range(d);
@@ -1178,12 +1178,11 @@ struct Box3 {
             SM[q] = sqrt(M[q]);
             return Vec<1>{{r * (r * M[q])}};
         });
-        // z = P r and gamma = r.z, then d = z
+        // z = P r and gamma = r.z
         x.spec_apply(d, R, SM, Z, nullptr, [=] __host__ __device__(Sc3 * s, double rz) {
             s->p_gamma = rz;
             s->p_beta = 0.0;
         });
-        x.p_dir_z(d, Z, DD, nullptr);
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->p_gamma_new = s->sum[0][0];   // r.Mr: the stopping quantity
             s->p_iter = 0;
@@ -1194,30 +1193,31 @@ struct Box3 {
             s->p_active = (conv || maxit <= 0) ? 0 : 1;
         });
         const int *gate = &sc->p_active;
-        for (int it = 0; it < maxit; it += CHUNK) {
-            for (int q = 0; q < CHUNK && it + q < maxit; q++) {
-                x.p_apply(d, CX, CY, CZ, DD, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
+        for (int it = 0, chunk = CHUNK; it < maxit; it += chunk, chunk = next_chunk(chunk)) {
+            for (int q = 0; q < chunk && it + q < maxit; q++) {
+                x.p_dir_apply(d, CX, CY, CZ, Z, D0, D1, PHI, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
                     s->p_alpha = s->p_gamma / (dAd + 1e-300);
                 });
-                x.p_update(d, PHI, R, DD, AD, M, gate, [=] __host__ __device__(Sc3 * s, double rMr) {
+                x.template p_resid<false>(d, R, AD, M, Z, gate, [=] __host__ __device__(Sc3 * s, double rMr) {
                     s->p_iter++;
                     s->p_gamma_new = rMr;
                     if (sqrt(rMr) < s->p_tol) s->p_active = 0;
                 });
-                // z = P r, r.z and the direction's coefficient, then d = z + beta d
+                // z = P r, r.z and the direction's coefficient
                 x.spec_apply(d, R, SM, Z, gate, [=] __host__ __device__(Sc3 * s, double g) {
                     s->p_beta = g / (s->p_gamma + 1e-300);
                     s->p_gamma = g;
                     if (s->p_iter >= s->p_maxit) s->p_active = 0;
                 });
-                x.p_dir_z(d, Z, DD, gate);
             }
             if (!x.read_int(gate)) break;
         }
         const int *ran = &sc->p_ran;
         const double count = (double)((long long)(d.NX - 1) * (d.NY - 1) * (d.NZ - 1));
         x.template reduce<1>(cr, ran, 0, [=] __host__ __device__(int i, int j, int k) {
-            return Vec<1>{{PHI[at(d, i, j, k)]}};
+            const long long q = at(d, i, j, k);
+            if (sc->p_iter > 0) PHI[q] += sc->p_alpha * ((sc->p_iter & 1) ? D1 : D0)[q];   // the last iteration's update
+            return Vec<1>{{PHI[q]}};
         });
         x.scalar(ran, [=] __host__ __device__(Sc3 * s) { s->p_avg = s->sum[0][0] / count; });
         x.cells(cr, ran, [=] __host__ __device__(int i, int j, int k) { PHI[at(d, i, j, k)] -= sc->p_avg; });
@@ -1237,7 +1237,7 @@ struct Box3 {
         const Dom3 d = this->d;
         Sc3 *sc = x.sc;
         const double *B = f[F3_PRHS], *M = f[F3_PM], *CX = f[F3_PCX], *CY = f[F3_PCY], *CZ = f[F3_PCZ];
-        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD];
+        double *PHI = f[F3_DP], *R = f[F3_PR], *D0 = f[F3_PD], *D1 = f[F3_PD2], *AD = f[F3_PAD], *Z = f[F3_PZ];
         const double tol = p.P_CG_ETOL;
         const int maxit = p.P_CG_MAXIT;
         const Range cr = cells_range(d);
@@ -1246,12 +1246,13 @@ struct Box3 {
             const double r = B[q] - p_apply_st(d, CX, CY, CZ, PHI, i, j, k);
             R[q] = r;
             const double z = r * M[q];
-            DD[q] = z;
+            Z[q] = z;
             return Vec<1>{{r * z}};
         });
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->p_gamma = s->sum[0][0];
             s->p_gamma_new = s->p_gamma;
+            s->p_beta = 0.0;
             s->p_iter = 0;
             s->p_maxit = maxit;
             s->p_tol = tol;
@@ -1260,19 +1261,18 @@ struct Box3 {
             s->p_active = (conv || maxit <= 0) ? 0 : 1;
         });
         const int *gate = &sc->p_active;
-        for (int it = 0; it < maxit; it += CHUNK) {
-            for (int q = 0; q < CHUNK && it + q < maxit; q++) {
-                // AD = A d and d.AD (the executor's streaming form of p_apply_st),
-                // then the step length from the finished sum
-                x.p_apply(d, CX, CY, CZ, DD, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
+        for (int it = 0, chunk = CHUNK; it < maxit; it += chunk, chunk = next_chunk(chunk)) {
+            for (int q = 0; q < chunk && it + q < maxit; q++) {
+                // phi += alpha d of the iteration before, d = z + beta d, AD = A d and
+                // d.AD, then the step length from the finished sum
+                x.p_dir_apply(d, CX, CY, CZ, Z, D0, D1, PHI, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
                     s->p_alpha = s->p_gamma / (dAd + 1e-30);
                 });
-                // phi += alpha d, r -= alpha AD and r.(M r), then the stopping test
-                // and the direction's coefficient
-                x.p_update(d, PHI, R, DD, AD, M, gate, [=] __host__ __device__(Sc3 * s, double rz) {
-                    s->sum[0][0] = rz;
+                // r -= alpha AD, z = M r and r.z, then the stopping test and the
+                // direction's coefficient
+                x.template p_resid<true>(d, R, AD, M, Z, gate, [=] __host__ __device__(Sc3 * s, double rz) {
                     s->p_iter++;
-                    s->p_gamma_new = s->sum[0][0];
+                    s->p_gamma_new = rz;
                     if (sqrt(s->p_gamma_new) < s->p_tol) {
                         s->p_active = 0;
                     } else {
@@ -1281,8 +1281,6 @@ struct Box3 {
                         if (s->p_iter >= s->p_maxit) s->p_active = 0;
                     }
                 });
-                // d = M r + beta d
-                x.p_dir(d, R, M, DD, gate);
             }
             if (!x.read_int(gate)) break;
         }
@@ -1290,7 +1288,9 @@ struct Box3 {
         const int *ran = &sc->p_ran;
         const double count = (double)((long long)(d.NX - 1) * (d.NY - 1) * (d.NZ - 1));
         x.template reduce<1>(cr, ran, 0, [=] __host__ __device__(int i, int j, int k) {
-            return Vec<1>{{PHI[at(d, i, j, k)]}};
+            const long long q = at(d, i, j, k);
+            if (sc->p_iter > 0) PHI[q] += sc->p_alpha * ((sc->p_iter & 1) ? D1 : D0)[q];   // the last iteration's update
+            return Vec<1>{{PHI[q]}};
         });
         x.scalar(ran, [=] __host__ __device__(Sc3 * s) { s->p_avg = s->sum[0][0] / count; });
         x.cells(cr, ran, [=] __host__ __device__(int i, int j, int k) { PHI[at(d, i, j, k)] -= sc->p_avg; });
