@@ -416,11 +416,8 @@ template <class A>
 int coop_launch(pvof_ctx *c, const void *fn, A &args, int n, int kind, int comp)
 {
     int nb = coop_blocks(c, n, kind);
-    // the solvers' counting grid barriers start from zero arrivals, the
-    // exchange slots of the one-cell-per-thread solvers from epoch zero
-    CK(cudaMemsetAsync(&c->scal->bar_arrivals, 0, sizeof(unsigned long long), c->stream));
-    if (n <= nb * COOP_THREADS)
-        CK(cudaMemsetAsync(c->partials, 0, SLOT_DOUBLES * (size_t)(nb + 1) * sizeof(double), c->stream));
+    // the solvers' exchange slots start from epoch zero
+    CK(cudaMemsetAsync(c->partials, 0, SLOT_DOUBLES * (size_t)(nb + 1) * sizeof(double), c->stream));
     return timed_launch(c, kind, comp, n, [&]() {
         void *params[] = {&args};
         return cudaLaunchCooperativeKernel(fn, dim3((unsigned)nb), dim3(COOP_THREADS), params, 0, c->stream);

@@ -19,126 +19,33 @@
 // The grid barriers are this file's own (not cooperative_groups::grid_group::
 // sync) so that their waits are bounded: if the other blocks never arrive
 // they record an error in DevScalars::error and every block leaves the
-// solver.  Ranges larger than one cell per resident thread count arrivals on
-// a counter that the host zeroes before each launch (grid_barrier_counted: a
-// fence, one atomic and the poll that sees the total).  Ranges of at most one
-// cell per resident thread keep the whole solve in registers and exchange
-// their sums through slots that are barrier and reduction in one
-// (grid_exchange).
+// solver.  The barrier is the exchange of the inner products' sums itself
+// (grid_exchange).  Ranges of at most one cell per resident thread keep the
+// whole solve in registers.
 #include "pvof_device.cuh"
 #include "pvof_kernels.cuh"
 
 namespace pvof {
 
-constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;
-
-// Grid barrier on a counter of arrivals that the host zeroes before the
-// launch: the g-th barrier of a launch is passed once the counter reaches
-// g * gridDim.x.  Each block's thread 0 publishes the block's writes
-// (block barrier, then a device-scope fence), adds its arrival without
-// waiting for the result and polls the counter; nothing is reset or bumped
-// after the last arrival, so the barrier costs a fence, one atomic and the
-// poll that sees the total.  Bounded: false (in every thread of the block)
-// when it gave up, with the error recorded.
-__device__ __noinline__ bool grid_barrier_counted(unsigned long long *arrivals, int *error, unsigned long long target)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned long long *va = arrivals;
-        volatile int *verr = error;
-        int good = 1;
-        __threadfence();
-        atomicAdd(arrivals, 1ull);
-        unsigned long long spins = 0;
-        while (*va < target) {
-            ++spins;
-            if ((spins & 1023ull) == 0 && (*verr != 0 || spins > BARRIER_SPIN_LIMIT)) {
-                atomicCAS(error, 0, 1);   // 1: a grid-wide solver's barrier
-                good = 0;
-                break;
-            }
-            if (spins > 4096) __nanosleep(64);
-        }
-        __threadfence();
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-// The counting barrier of one launch: the launch's g-th call waits for
-// g * gridDim.x arrivals.
-struct CountedSync {
-    DevScalars *s;
-    unsigned long long target;
-    __device__ bool sync()
-    {
-        target += gridDim.x;
-        return grid_barrier_counted(&s->bar_arrivals, &s->error, target);
-    }
-};
-
-// sum of v over the block (1D blocks, multiple of 32 threads)
-__device__ double block_sum(double v)
-{
-    __shared__ double sh[32];
-    __shared__ double res;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        double w = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) w += __shfl_down_sync(0xffffffffu, w, o);
-        if (lane == 0) res = w;
-    }
-    __syncthreads();
-    return res;
-}
-
-// Sum of the per-block partials, identical in every block.  Each reduction
-// uses its own slot of the partials buffer; a slot is rewritten only after at
-// least one more barrier has passed since every block read it.
-__device__ double grid_total(const double *part)
-{
-    __shared__ double res;
-    if (threadIdx.x < 32) {
-        double v = 0.0;
-        for (unsigned q = threadIdx.x; q < gridDim.x; q += 32) v += part[q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (threadIdx.x == 0) res = v;
-    }
-    __syncthreads();
-    double r = res;
-    __syncthreads();
-    return r;
-}
-
-__device__ __forceinline__ void put_partial(double *part, double v)
-{
-    double s = block_sum(v);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
+constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;   // polls of one wait
 
 // Grid-wide sum and barrier in one: every block publishes its partial sums in
 // a slot of its own, tagged with the number of the exchange (the epoch).  On
 // at most 32 blocks every block polls all slots until they carry that tag; on
 // more, block 0 does and publishes the totals in one more slot, which the
 // other blocks poll (all blocks polling all slots crowds the few L2 lines the
-// slots lie in).  One or two one-way trips through L2 replace
-// grid_barrier_counted's atomic, its poll and the load of the partials behind
-// it.  Measured, B200, us per exchange without and with PUBLISH: 9 blocks
-// of 512 threads 0.97 and 1.9, counted barrier and partials 2.5; 227 blocks
-// 2.1 and 3.2, every block polling 4.4 and 5.3, counted 6.3.
+// slots lie in).  One or two one-way trips through L2; a barrier that counts
+// arrivals and a load of the partials behind it take three.  Measured, B200,
+// us per exchange without and with PUBLISH: 9 blocks of 512 threads 0.97 and
+// 1.9, counting barrier and partials 2.5; 227 blocks 2.1 and 3.2, every block
+// polling 4.4 and 5.3, counting 6.3.
 // A slot holds each double as two words of 32 value bits and the 32-bit
 // epoch, so a word is valid by itself and the two need not arrive together.
 // Two buffers alternate: a block writes epoch e + 2 only after it has the
 // totals of e + 1, which need every block's e + 1, published after it read e.
 // The host zeroes the slots before each launch; epochs start at 1.  The sums
-// are taken in put_partial's and grid_total's order, so the totals are theirs
-// bit for bit.
+// are taken in a fixed order (a tree in the block, then the blocks by lane), so
+// every block has the same totals and runs repeat bit for bit.
 // PUBLISH: the block's earlier stores to global memory are visible to every
 // block after the exchange (else only the sums are exchanged): a fence before
 // the block's slot is written, acquiring loads once a slot has been seen, and
@@ -286,15 +193,13 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
-    CountedSync gs{A.scal, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
     const Range R{0, 0, NX - 1, (NX - 1) * (NY - 1)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double nk = (double)d.nk;
-    double *part0 = A.partials, *part1 = A.partials + gridDim.x;
-    double *part2 = A.partials + 2 * gridDim.x, *part3 = A.partials + 3 * gridDim.x;
 
     // L(L(f)) at (i,j) for a field given at sources: lap of the ghost-updated
-    // Laplacian of the ghost-updated f (VOF_DIFFUSE_compute_laplacian twice)
+    // Laplacian of the ghost-updated f (VOF_DIFFUSE_compute_laplacian twice).
     auto bilap = [&](int i, int j, auto fsrc) {
         auto fv = [&](int a, int b) {
             int si, sj;
@@ -325,12 +230,11 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
         sbb += m * bv * bv;
         srr += m * rv * rv;
     }
-    put_partial(part0, sbb);
-    put_partial(part1, srr);
-    if (!gs.sync()) return;
-    double rhs_norm = sqrt(nk * grid_total(part0));
+    double both[2] = {sbb, srr}, one[1];
+    if (!grid_exchange<2, true>(sl, both)) return;
+    double rhs_norm = sqrt(nk * both[0]);
     if (rhs_norm < 1e-30) rhs_norm = 1.0;
-    double rz = nk * grid_total(part1);
+    double rz = nk * both[1];
     double rel = sqrt(rz) / rhs_norm;
     int iter = 0;
     if (rel < A.tol) {
@@ -363,9 +267,10 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
         }
         if (!first) { double *t = pcur; pcur = pnxt; pnxt = t; }
         first = false;
-        put_partial(part2, spap);
-        if (!gs.sync()) return;
-        double pAp = nk * grid_total(part2);
+        // the update reads its own cells' p and Ap only: the sum alone
+        one[0] = spap;
+        if (!grid_exchange<1, false>(sl, one)) return;
+        double pAp = nk * one[0];
         if (fabs(pAp) < 1e-30) break;
         double alpha = rz / pAp;
         double srr2 = 0.0;
@@ -377,10 +282,10 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
             AT_(A.r, i, j) = rv;
             srr2 += d.m.wx[i] * d.m.wy[j] * d.wz * rv * rv;
         }
-        put_partial(part3, srr2);
-        if (!gs.sync()) return;
+        one[0] = srr2;
+        if (!grid_exchange<1, true>(sl, one)) return;
         ++iter;
-        double rr = nk * grid_total(part3);
+        double rr = nk * one[0];
         rel = sqrt(rr) / rhs_norm;
         if (rel < A.tol) break;
         double rz_new = rr;  // z == r: the same weighted sum
@@ -514,12 +419,10 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
-    CountedSync gs{A.scal, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
     const Range R{A.i0, A.j0, A.i1 - A.i0, (A.i1 - A.i0) * (A.j1 - A.j0)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double EPS = 1e-14;
-    double *part0 = A.partials, *part1 = A.partials + gridDim.x;
-    double *part2 = A.partials + 2 * gridDim.x, *part3 = A.partials + 3 * gridDim.x;
     auto active = [&](int a, int b) { return a >= A.i0 && a < A.i1 && b >= A.j0 && b < A.j1; };
 
     double srz = 0.0;
@@ -537,9 +440,9 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
         AT_(A.z, i, j) = dv;
         srz += rv * dv;
     }
-    put_partial(part0, srz);
-    if (!gs.sync()) return;
-    double rz = grid_total(part0);
+    double one[1] = {srz}, both[2];
+    if (!grid_exchange<1, true>(sl, one)) return;
+    double rz = one[0];
     double RMS = 0.0, beta = 0.0;
     int iters = 0;
     double *dcur = A.dir, *dnxt = A.dir2;
@@ -579,10 +482,9 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
         }
         if (!first) { double *t = dcur; dcur = dnxt; dnxt = t; }
         first = false;
-        put_partial(part1, sdad);
-        if (!gs.sync()) return;
-        double dAd = grid_total(part1);
-        double alpha = rz / (dAd + A.step_eps);
+        one[0] = sdad;   // the update reads its own cells' d and Ad only
+        if (!grid_exchange<1, false>(sl, one)) return;
+        double alpha = rz / (one[0] + A.step_eps);
         double s0 = 0.0, s1 = 0.0;
         for (int q = tid; q < R.n; q += nth) {
             int i, j;
@@ -595,10 +497,10 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
             s0 += ri * ri / dg;
             s1 += ri * ri;
         }
-        put_partial(part2, s0);
-        put_partial(part3, s1);
-        if (!gs.sync()) return;
-        double rz_new = grid_total(part2), rr = grid_total(part3);
+        both[0] = s0;
+        both[1] = s1;
+        if (!grid_exchange<2, true>(sl, both)) return;
+        double rz_new = both[0], rr = both[1];
         RMS = sqrt(A.in_tot * rr);
         if (RMS < A.tol) break;
         beta = rz_new / (rz + A.step_eps);
@@ -725,14 +627,13 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     const int P = d.P, NX = d.NX, NY = d.NY;
     const Range R{0, 0, NX - 1, (NX - 1) * (NY - 1)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    double *part0 = A.partials, *part1 = A.partials + gridDim.x, *part2 = A.partials + 2 * gridDim.x;
     // sources of the neighbours beyond the ends of the solve range
     const int xw = A.mp.x.src[NG - 1], xe = A.mp.x.src[NX - 1 + NG];
     const int ys = A.mp.y.src[NG - 1], yn = A.mp.y.src[NY - 1 + NG];
     const double *__restrict__ rho = A.rho;
     const double *__restrict__ bx = A.bx;
     const double *__restrict__ by = A.by;
-    CountedSync cs{A.scal, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
     if (!PAIR && R.n <= nth) {   // one cell per thread
         cg_pressure_resident(A, R);
         return;
@@ -753,9 +654,9 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         AT_(A.z, i, j) = z;
         sg += rv * z;
     }
-    put_partial(part0, sg);
-    if (!cs.sync()) return;
-    double gamma = grid_total(part0), gamma_new = 0.0, beta = 0.0;
+    double one[1] = {sg};
+    if (!grid_exchange<1, true>(sl, one)) return;
+    double gamma = one[0], gamma_new = 0.0, beta = 0.0;
     if (sqrt(gamma) < A.tol) {
         if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = 0; A.scal->p_res = sqrt(gamma); }
         return;
@@ -891,9 +792,9 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         }
         if (!first) { double *t = dcur; dcur = dnxt; dnxt = t; }
         first = false;
-        put_partial(part1, sdad);
-        if (!cs.sync()) return;
-        alpha = gamma / (grid_total(part1) + 1e-30);
+        one[0] = sdad;   // the update reads its own cells' Ad only
+        if (!grid_exchange<1, false>(sl, one)) return;
+        alpha = gamma / (one[0] + 1e-30);
         double sgn = 0.0;
         if (PAIR)
             for (int p = tid; p < Np; p += nth) update_pair(p, alpha, sgn);
@@ -922,9 +823,9 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
                 sgn += rv * z;
             }
         }
-        put_partial(part2, sgn);
-        if (!cs.sync()) return;
-        gamma_new = grid_total(part2);
+        one[0] = sgn;
+        if (!grid_exchange<1, true>(sl, one)) return;
+        gamma_new = one[0];
         if (sqrt(gamma_new) < A.tol) break;
         beta = gamma_new / (gamma + 1e-30);
         gamma = gamma_new;
@@ -939,9 +840,9 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
         if (pending) AT_(A.phi, i, j) += alpha * AT_(dcur, i, j);
         ssum += AT_(A.phi, i, j);
     }
-    put_partial(part0, ssum);
-    if (!cs.sync()) return;
-    double avg = grid_total(part0) / (double)R.n;
+    one[0] = ssum;
+    if (!grid_exchange<1, false>(sl, one)) return;
+    double avg = one[0] / (double)R.n;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);

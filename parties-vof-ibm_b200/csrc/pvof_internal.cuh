@@ -107,7 +107,6 @@ struct DevScalars {
     double cnn_ms[2];   // mean squares of the network's rhs and phi_prev inputs
     double mass;
     int error;          // non-zero: a grid barrier gave up (see pvof_cg.cu)
-    unsigned long long bar_arrivals;   // arrivals at the counting grid barrier, zeroed before each launch
 };
 
 // launch shape of a strip solver: threads per CTA (0: the range does not fit)
@@ -149,7 +148,7 @@ struct Ctx {
     int *map_src_mem;
     double *map_mul_mem;
     BcMap maps[BK_COUNT];
-    double *partials;        // per-block partial sums (SLOT_DOUBLES per block)
+    double *partials;        // per-block partial sums and exchange slots (SLOT_DOUBLES per block and one more)
     DevScalars *scal;        // device scalars
     DevScalars *scal_host;   // pinned host mirror
     double *host_plane;      // pinned staging plane for uploads/downloads

@@ -37,9 +37,8 @@ struct VelArgs {
     double *ft = nullptr, *mc = nullptr;   // time-term and corner-viscosity planes (k_cg_velocity)
 };
 
-// doubles per block (and one more) of the partial sums: four sums of the
-// grid-stride solvers, or two buffers of two-value exchange slots (two words
-// per value) of the one-cell-per-thread ones
+// doubles per block (and one more) of the grid-wide solvers' exchange slots: two
+// buffers of two values, two words per value
 constexpr size_t SLOT_DOUBLES = 8;
 
 struct PresArgs {
