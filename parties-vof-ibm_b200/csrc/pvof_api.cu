@@ -898,20 +898,16 @@ int p_solve_spectral(pvof_ctx *c)
         if (c->spec_blocks <= 0) return set_err(PVOF_ECUDA, "the spectral pressure solve needs a cooperative launch");
         std::vector<double> tw, tri;
         spec_tables(N, M, idx2, idy2, tw, tri);
-        const size_t parts = 3 * (size_t)c->spec_blocks;
+        const size_t parts = spec_slot_doubles(c->spec_blocks);
         std::vector<double> h(tw);
         h.resize(h.size() + parts, 0.0);
         h.insert(h.end(), tri.begin(), tri.end());
         h.resize(h.size() + 3 * c->plane_elems, 0.0);   // the face coefficients and weight roots of a solve
-        if (cudaMalloc(&c->spec_mem, h.size() * sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&c->spec_s, sizeof(SpecScal)) != cudaSuccess)
+        if (cudaMalloc(&c->spec_mem, h.size() * sizeof(double)) != cudaSuccess)
             return set_err(PVOF_ENOMEM, "allocating the spectral preconditioner");
         // on the context's (non-blocking) stream, so the solve's launches are
-        // ordered after them; a copy or memset on the legacy default stream
-        // is not, and a zeroing of the barrier state landing in the middle of
-        // the first solve erased arrivals (a grid barrier timeout)
+        // ordered after it; a copy on the legacy default stream is not
         CK(cudaMemcpyAsync(c->spec_mem, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemsetAsync(c->spec_s, 0, sizeof(SpecScal), c->stream));
     }
     SpecArgs A;
     A.d = d;
@@ -926,7 +922,7 @@ int p_solve_spectral(pvof_ctx *c)
     A.hat = S(c, SC_P_HAT);
     A.tw = reinterpret_cast<const double2 *>(c->spec_mem);
     A.part = c->spec_mem + N;
-    A.tri = A.part + 3 * (size_t)c->spec_blocks;
+    A.tri = A.part + spec_slot_doubles(c->spec_blocks);
     {
         const int NW = N / 2 + 1;
         const int P = M / 2 < 32 ? M / 2 : 32;   // spec_tables' chunk rule: P chunks, K the longest
@@ -945,7 +941,6 @@ int p_solve_spectral(pvof_ctx *c)
     A.fscale = c->spec_fscale;
     A.tol = c->p.P_CG_ETOL;
     A.maxit = c->p.P_CG_MAXIT;
-    A.s = c->spec_s;
     A.scal = c->scal;
     TRY(timed_launch(c, PVOF_SOLVER_PRESSURE, 0, N * M, [&]() {
         return spec_launch_pcg(A, c->spec_blocks, S(c, SC_P_D), S(c, SC_P_D2), c->stream);
@@ -1030,7 +1025,6 @@ int read_scalars(pvof_ctx *c)
     if (c->scal_host->error) {
         const int code = c->scal_host->error;
         CK(cudaMemsetAsync(c->scal, 0, sizeof(DevScalars), c->stream));
-        if (c->spec_s) CK(cudaMemsetAsync(c->spec_s, 0, sizeof(SpecScal), c->stream));
         CK(cudaStreamSynchronize(c->stream));
         return set_err(PVOF_ECUDA, code == 4 ? "advection tile load timed out"
                                    : code == 5 ? "cluster solver: an exchange between its blocks timed out"
@@ -1958,10 +1952,11 @@ int pvof_create(const pvof_grid_desc *grid, const pvof_params *params, int devic
     }
     ob = std::min(o1, std::min(o2, o3));
     if (ob < 1) return fail(PVOF_ECUDA, "persistent solver kernels do not fit on an SM");
-    c->coop_blocks_of[PVOF_SOLVER_BIHARMONIC] = o1 * nsm;   // each as many as it keeps co-resident
-    c->coop_blocks_of[PVOF_SOLVER_VELOCITY] = o2 * nsm;
-    c->coop_blocks_of[PVOF_SOLVER_PRESSURE] = o3 * nsm;
-    c->coop_blocks = std::max(o1, std::max(o2, o3)) * nsm;
+    // each as many as it keeps co-resident and exchanges sums among
+    c->coop_blocks_of[PVOF_SOLVER_BIHARMONIC] = std::min(o1 * nsm, SLOT_BLOCKS);
+    c->coop_blocks_of[PVOF_SOLVER_VELOCITY] = std::min(o2 * nsm, SLOT_BLOCKS);
+    c->coop_blocks_of[PVOF_SOLVER_PRESSURE] = std::min(o3 * nsm, SLOT_BLOCKS);
+    c->coop_blocks = *std::max_element(c->coop_blocks_of, c->coop_blocks_of + 3);
     c->coop_threads = COOP_THREADS;
     // cluster-resident solvers when the solve ranges fit one cluster
     // (pvof_set_cluster_solvers selects the grid-wide forms instead)
@@ -2029,7 +2024,6 @@ int pvof_destroy(pvof_ctx *c)
         if (g.exec) cudaGraphExecDestroy(g.exec);
     if (c->fft_coef) cudaFree(c->fft_coef);
     if (c->spec_mem) cudaFree(c->spec_mem);
-    if (c->spec_s) cudaFree(c->spec_s);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return PVOF_OK;

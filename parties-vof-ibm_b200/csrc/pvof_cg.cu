@@ -23,145 +23,10 @@
 // (grid_exchange).  Ranges of at most one cell per resident thread keep the
 // whole solve in registers.
 #include "pvof_device.cuh"
+#include "pvof_exchange.cuh"
 #include "pvof_kernels.cuh"
 
 namespace pvof {
-
-constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;   // polls of one wait
-
-// Grid-wide sum and barrier in one: every block publishes its partial sums in
-// a slot of its own, tagged with the number of the exchange (the epoch).  On
-// at most 32 blocks every block polls all slots until they carry that tag; on
-// more, block 0 does and publishes the totals in one more slot, which the
-// other blocks poll (all blocks polling all slots crowds the few L2 lines the
-// slots lie in).  One or two one-way trips through L2; a barrier that counts
-// arrivals and a load of the partials behind it take three.  Measured, B200,
-// us per exchange without and with PUBLISH: 9 blocks of 512 threads 0.97 and
-// 1.9, counting barrier and partials 2.5; 227 blocks 2.1 and 3.2, every block
-// polling 4.4 and 5.3, counting 6.3.
-// A slot holds each double as two words of 32 value bits and the 32-bit
-// epoch, so a word is valid by itself and the two need not arrive together.
-// Two buffers alternate: a block writes epoch e + 2 only after it has the
-// totals of e + 1, which need every block's e + 1, published after it read e.
-// The host zeroes the slots before each launch; epochs start at 1.  The sums
-// are taken in a fixed order (a tree in the block, then the blocks by lane), so
-// every block has the same totals and runs repeat bit for bit.
-// PUBLISH: the block's earlier stores to global memory are visible to every
-// block after the exchange (else only the sums are exchanged): a fence before
-// the block's slot is written, acquiring loads once a slot has been seen, and
-// a fence in block 0 before the totals.  False, in every thread of the block,
-// when the bounded wait gave up.
-struct Slots {
-    unsigned long long *w;   // two buffers of gridDim.x + 1 slots
-    int *error;
-    unsigned epoch;
-};
-
-constexpr unsigned ALL_POLL_BLOCKS = 32;
-constexpr int SLOT_BLOCKS = 512;   // most blocks: one slot per thread of block 0
-
-__device__ __forceinline__ void slot_put(unsigned long long *p, double v, unsigned e)
-{
-    const unsigned long long x = (unsigned long long)__double_as_longlong(v), tag = (unsigned long long)e << 32;
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"((x & 0xffffffffull) | tag), "l"((x >> 32) | tag)
-                 : "memory");
-}
-
-// waits (bounded) for epoch e in slot p
-template <bool ACQUIRE>
-__device__ __forceinline__ bool slot_get(const unsigned long long *p, unsigned e, double &v, int *error)
-{
-    unsigned long long lo, hi, spins = 0;
-    for (;;) {
-        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
-        if ((unsigned)(lo >> 32) == e && (unsigned)(hi >> 32) == e) break;
-        ++spins;
-        if ((spins & 1023ull) == 0 && (*(volatile int *)error != 0 || spins > BARRIER_SPIN_LIMIT)) {
-            atomicCAS(error, 0, 1);   // 1: a grid-wide solver's barrier
-            return false;
-        }
-        if (spins > 4096) __nanosleep(64);
-    }
-    if (ACQUIRE) {
-        unsigned long long seen;
-        asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(seen) : "l"(p) : "memory");
-    }
-    v = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
-    return true;
-}
-
-template <int NV, bool PUBLISH>
-__device__ __forceinline__ bool grid_exchange(Slots &sl, double (&v)[NV])
-{
-    __shared__ double wsum[32][NV], vals[NV][SLOT_BLOCKS], total[NV];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned nb = gridDim.x, e = ++sl.epoch;
-    unsigned long long *buf = sl.w + (size_t)(e & 1u) * (nb + 1) * 2 * NV;
-    int good = 1;
-#pragma unroll
-    for (int n = 0; n < NV; n++)
-        for (int o = 16; o > 0; o >>= 1) v[n] += __shfl_down_sync(0xffffffffu, v[n], o);
-    if (lane == 0)
-#pragma unroll
-        for (int n = 0; n < NV; n++) wsum[warp][n] = v[n];
-    __syncthreads();
-    if (warp == 0) {
-        double b[NV];
-#pragma unroll
-        for (int n = 0; n < NV; n++) {
-            b[n] = lane < (int)(blockDim.x >> 5) ? wsum[lane][n] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) b[n] += __shfl_down_sync(0xffffffffu, b[n], o);
-        }
-        if (lane == 0) {
-            if (PUBLISH) __threadfence();
-#pragma unroll
-            for (int n = 0; n < NV; n++) slot_put(buf + ((size_t)blockIdx.x * NV + n) * 2, b[n], e);
-        }
-        __syncwarp();
-    }
-    if (nb <= ALL_POLL_BLOCKS) {
-        if (warp == 0) {
-#pragma unroll
-            for (int n = 0; n < NV; n++) {
-                double t = 0.0;
-                if (lane < (int)nb && !slot_get<PUBLISH>(buf + ((size_t)lane * NV + n) * 2, e, t, sl.error)) good = 0;
-                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-                if (lane == 0) total[n] = t;
-            }
-        }
-    } else if (blockIdx.x == 0) {
-        for (unsigned q = threadIdx.x; q < nb; q += blockDim.x)
-#pragma unroll
-            for (int n = 0; n < NV; n++)
-                if (!slot_get<PUBLISH>(buf + ((size_t)q * NV + n) * 2, e, vals[n][q], sl.error)) good = 0;
-        __syncthreads();
-        if (warp == 0) {
-            double t[NV];
-#pragma unroll
-            for (int n = 0; n < NV; n++) {
-                t[n] = 0.0;
-                for (unsigned q = lane; q < nb; q += 32) t[n] += vals[n][q];
-                for (int o = 16; o > 0; o >>= 1) t[n] += __shfl_xor_sync(0xffffffffu, t[n], o);
-            }
-            if (lane == 0) {
-                if (PUBLISH) __threadfence();
-#pragma unroll
-                for (int n = 0; n < NV; n++) {
-                    slot_put(buf + ((size_t)nb * NV + n) * 2, t[n], e);
-                    total[n] = t[n];
-                }
-            }
-        }
-    } else if (threadIdx.x == 0) {
-#pragma unroll
-        for (int n = 0; n < NV; n++)
-            if (!slot_get<PUBLISH>(buf + ((size_t)nb * NV + n) * 2, e, total[n], sl.error)) good = 0;
-    }
-    good = __syncthreads_and(good);
-#pragma unroll
-    for (int n = 0; n < NV; n++) v[n] = total[n];
-    return good != 0;
-}
 
 struct Range {
     int i0, j0, w, n;
@@ -189,11 +54,11 @@ __device__ __forceinline__ void src_of(const BcMap &m, int NX, int NY, int i, in
 // evaluated on the fly (with the scalar ghost update in between), so one
 // iteration needs two grid barriers.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
+__global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
-    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
     const Range R{0, 0, NX - 1, (NX - 1) * (NY - 1)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double nk = (double)d.nk;
@@ -242,12 +107,12 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
         return;
     }
     double *pcur = A.p1, *pnxt = A.p2;
-    double beta = 0.0;
-    bool first = true;
+    double beta = 0.0, alpha = 0.0;
+    bool first = true, pending = false;   // pending: x += alpha p_cur still to be applied
     while (iter < A.maxit) {
         // p = z + beta p (z = r); Ap = a_dt p + bih L(L(p))
         double spap = 0.0;
-        const double bt = beta;
+        const double bt = beta, al = alpha;
         const double *pold = pcur;
         for (int q = tid; q < R.n; q += nth) {
             int i, j;
@@ -257,8 +122,10 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
                 pv = AT_(pold, i, j);
                 l2 = bilap(i, j, [&](int a, int b) { return AT_(pold, a, b); });
             } else {
-                pv = AT_(A.r, i, j) + bt * AT_(pold, i, j);
+                const double po = AT_(pold, i, j);
+                pv = AT_(A.r, i, j) + bt * po;
                 AT_(pnxt, i, j) = pv;
+                AT_(A.x, i, j) += al * po;   // the update of the iteration before
                 l2 = bilap(i, j, [&](int a, int b) { return AT_(A.r, a, b) + bt * AT_(pold, a, b); });
             }
             double ap = A.a_dt * pv + A.bih * l2;
@@ -267,20 +134,33 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
         }
         if (!first) { double *t = pcur; pcur = pnxt; pnxt = t; }
         first = false;
-        // the update reads its own cells' p and Ap only: the sum alone
+        // the update reads its own cells' Ap only: the sum alone
         one[0] = spap;
+        pending = false;
         if (!grid_exchange<1, false>(sl, one)) return;
         double pAp = nk * one[0];
         if (fabs(pAp) < 1e-30) break;
-        double alpha = rz / pAp;
+        alpha = rz / pAp;
+        pending = true;
         double srr2 = 0.0;
-        for (int q = tid; q < R.n; q += nth) {
-            int i, j;
+        for (int q = tid; q < R.n; q += 2 * nth) {   // two cells per trip
+            const int q1 = q + nth;
+            const bool two = q1 < R.n;
+            int i, j, i1 = 0, j1 = 0;
             R.ij(q, i, j);
-            AT_(A.x, i, j) += alpha * AT_(pcur, i, j);
-            double rv = AT_(A.r, i, j) - alpha * AT_(A.Ap, i, j);
+            const double r0 = AT_(A.r, i, j), a0 = AT_(A.Ap, i, j);
+            double r1 = 0.0, a1 = 0.0;
+            if (two) {
+                R.ij(q1, i1, j1);
+                r1 = AT_(A.r, i1, j1); a1 = AT_(A.Ap, i1, j1);
+            }
+            const double rv = r0 - alpha * a0, rw = r1 - alpha * a1;
             AT_(A.r, i, j) = rv;
             srr2 += d.m.wx[i] * d.m.wy[j] * d.wz * rv * rv;
+            if (two) {
+                AT_(A.r, i1, j1) = rw;
+                srr2 += d.m.wx[i1] * d.m.wy[j1] * d.wz * rw * rw;
+            }
         }
         one[0] = srr2;
         if (!grid_exchange<1, true>(sl, one)) return;
@@ -292,6 +172,12 @@ __global__ void __launch_bounds__(512) k_cg_biharmonic(BihArgs A)
         beta = rz_new / (rz + 1e-30);
         rz = rz_new;
     }
+    if (pending)
+        for (int q = tid; q < R.n; q += nth) {
+            int i, j;
+            R.ij(q, i, j);
+            AT_(A.x, i, j) += alpha * AT_(pcur, i, j);
+        }
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->ch_iters = iter; A.scal->ch_rel = rel; }
 }
 
@@ -319,7 +205,7 @@ __global__ void __launch_bounds__(512, 2) k_cg_velocity_res(VelArgs A)
     int i = A.i0, j = A.j0;
     if (on) R.ij(q, i, j);
     const int comp = A.comp;
-    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
     double r = 0.0, dg = 1.0, ft = 0.0, x = 0.0, z = 0.0;
     double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;   // viscosities of the x+, x-, y+, y- faces
     ptrdiff_t off[4];
@@ -415,11 +301,11 @@ __global__ void __launch_bounds__(512, 2) k_cg_velocity_res(VelArgs A)
 // Velocity_solve_cg (Eulerian/lsolver/msolve_cg.c:525-722): Jacobi PCG with
 // the RMS residual stop, one velocity component.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
+__global__ void __launch_bounds__(512, 2) k_cg_velocity(VelArgs A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
-    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
     const Range R{A.i0, A.j0, A.i1 - A.i0, (A.i1 - A.i0) * (A.j1 - A.j0)};
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double EPS = 1e-14;
@@ -447,11 +333,12 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
     int iters = 0;
     double *dcur = A.dir, *dnxt = A.dir2;
     bool first = true;
+    double alpha = 0.0;   // the step of the update x += alpha d_cur still to be applied
     while (iters < A.maxit) {
         iters++;
         // d = M^-1 r + beta d, Ad = A d with the VEL_TYPE_CG ghost update of d
         double sdad = 0.0;
-        const double bt = beta;
+        const double bt = beta, al = alpha;
         const double *dold = dcur;
         for (int q = tid; q < R.n; q += nth) {
             int i, j;
@@ -477,25 +364,39 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
                     return mul * (AT_(A.z, si, sj) + bt * AT_(dold, si, sj));
                 });
             }
+            if (!first) AT_(A.x, i, j) += al * AT_(dold, i, j);   // the update of the iteration before
             AT_(A.Ad, i, j) = ad;
             sdad += dv * ad;
         }
         if (!first) { double *t = dcur; dcur = dnxt; dnxt = t; }
         first = false;
-        one[0] = sdad;   // the update reads its own cells' d and Ad only
+        one[0] = sdad;   // the update reads its own cells' Ad only
         if (!grid_exchange<1, false>(sl, one)) return;
-        double alpha = rz / (one[0] + A.step_eps);
+        alpha = rz / (one[0] + A.step_eps);
         double s0 = 0.0, s1 = 0.0;
-        for (int q = tid; q < R.n; q += nth) {
-            int i, j;
+        // two cells per trip, their loads before either's stores
+        for (int q = tid; q < R.n; q += 2 * nth) {
+            const int q1 = q + nth;
+            const bool two = q1 < R.n;
+            int i, j, i1 = 0, j1 = 0;
             R.ij(q, i, j);
-            AT_(A.x, i, j) += alpha * AT_(dcur, i, j);
-            double ri = AT_(A.r, i, j) - alpha * AT_(A.Ad, i, j);
+            const double r0 = AT_(A.r, i, j), a0 = AT_(A.Ad, i, j), g0 = AT_(A.diag, i, j);
+            double r1 = 0.0, a1 = 0.0, g1 = 1.0;
+            if (two) {
+                R.ij(q1, i1, j1);
+                r1 = AT_(A.r, i1, j1); a1 = AT_(A.Ad, i1, j1); g1 = AT_(A.diag, i1, j1);
+            }
+            const double ri = r0 - alpha * a0, rj = r1 - alpha * a1;
             AT_(A.r, i, j) = ri;
-            double dg = AT_(A.diag, i, j);
-            AT_(A.z, i, j) = ri / dg;
-            s0 += ri * ri / dg;
+            AT_(A.z, i, j) = ri / g0;
+            s0 += ri * ri / g0;
             s1 += ri * ri;
+            if (two) {
+                AT_(A.r, i1, j1) = rj;
+                AT_(A.z, i1, j1) = rj / g1;
+                s0 += rj * rj / g1;
+                s1 += rj * rj;
+            }
         }
         both[0] = s0;
         both[1] = s1;
@@ -506,6 +407,12 @@ __global__ void __launch_bounds__(512) k_cg_velocity(VelArgs A)
         beta = rz_new / (rz + A.step_eps);
         rz = rz_new;
     }
+    if (!first)
+        for (int q = tid; q < R.n; q += nth) {
+            int i, j;
+            R.ij(q, i, j);
+            AT_(A.x, i, j) += alpha * AT_(dcur, i, j);
+        }
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->vel_iters[A.comp] = iters; A.scal->vel_rms[A.comp] = RMS; }
 }
 
@@ -546,7 +453,7 @@ __device__ __forceinline__ void cg_pressure_resident(const PresArgs &A, const Ra
     const bool on = q < R.n;
     int i = 0, j = 0;
     if (on) R.ij(q, i, j);
-    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
     double r = 0.0, m = 0.0, z = 0.0, ph = 0.0, rw = 1.0;
     double cxm = 0.0, cxp = 0.0, cym = 0.0, cyp = 0.0;
     const ptrdiff_t cC = (ptrdiff_t)j * P + i;
@@ -633,7 +540,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     const double *__restrict__ rho = A.rho;
     const double *__restrict__ bx = A.bx;
     const double *__restrict__ by = A.by;
-    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, 0};
+    Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
     if (!PAIR && R.n <= nth) {   // one cell per thread
         cg_pressure_resident(A, R);
         return;

@@ -190,7 +190,6 @@ struct Ctx {
     pvof3::Handle *h3;       // the 3D mode's state (PVOF_GEOM_3D); null for the 2D modes
     double *fft_coef;        // the FFT Poisson solver's tables (p_solve_fft)
     double *spec_mem;        // spectral pressure preconditioner: twiddles, block sums, reduction tables
-    struct SpecScal *spec_s; // its grid barrier state
     double spec_fscale;      // dy^2 / N
     int spec_blocks;         // blocks of its cooperative launch
     double sol_ms[3];

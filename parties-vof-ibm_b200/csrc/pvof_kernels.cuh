@@ -40,6 +40,7 @@ struct VelArgs {
 // doubles per block (and one more) of the grid-wide solvers' exchange slots: two
 // buffers of two values, two words per value
 constexpr size_t SLOT_DOUBLES = 8;
+constexpr int SLOT_BLOCKS = 320;   // most blocks of an exchange (two per SM of a B200 are 296)
 
 struct PresArgs {
     Dom d;
@@ -55,11 +56,8 @@ struct PresArgs {
 };
 
 // spectral-preconditioned pressure PCG (pvof_spec.cu)
-struct SpecScal {
-    unsigned arrivals;   // arrivals at the solve's grid barriers, zeroed before each launch
-};
-
 constexpr int SPEC_PT = 1024;        // threads per block of the cooperative solve
+constexpr size_t spec_slot_doubles(int blocks) { return 4 * ((size_t)blocks + 1); }
 
 struct SpecArgs {
     Dom d;
@@ -75,8 +73,7 @@ struct SpecArgs {
     double fscale;            // dy^2 / N
     double tol;
     int maxit;
-    double *part;             // per-block sums, three slots of gridDim entries
-    SpecScal *s;
+    double *part;             // exchange slots, spec_slot_doubles(blocks)
     DevScalars *scal;
 };
 
@@ -156,11 +153,11 @@ struct HostMap {
     std::vector<double> xmul, ymul;
 };
 
+
 // the two velocity components of one launch: cluster q solves c[q]
 struct VelPair {
     VelArgs c[2];
 };
-
 
 StripPlan cgs_pressure_setup(int NX, int NY, int axisym, const HostMap &mp);
 cudaError_t cgs_pressure_launch(const PresArgs &A, const StripPlan &plan, cudaStream_t stream);

@@ -46,18 +46,18 @@
 //
 // The whole solve is ONE cooperative launch: blocks of SPEC_PT threads, eight
 // 128-thread row groups in the row phases, eight warps of one tridiagonal
-// system each per block in the solve phase, four grid barriers per iteration (after the
-// matrix-vector product, the update with its forward transforms, the
-// tridiagonal solves, the inverse transforms), one more per solve after the
-// solve's constants (face coefficients, weight roots).  Every block adds the
-// per-block sums in block order, so all of them take the same decisions.  The
-// grid barrier resets itself (the last arriver zeroes the count and advances
-// a generation); its wait is bounded (on timeout the error flag in DevScalars
-// is set and every block leaves).
+// system each per block in the solve phase, four grid-wide exchanges per
+// iteration (grid_exchange: after the matrix-vector product, the update with
+// its forward transforms, the tridiagonal solves, the inverse transforms), one
+// more per solve after the solve's constants (face coefficients, weight
+// roots).  All blocks get the same sums, so all of them take the same
+// decisions; the waits are bounded (on timeout the error flag in DevScalars is
+// set and every block leaves).
 #include <cmath>
 #include <vector>
 
 #include "pvof_device.cuh"
+#include "pvof_exchange.cuh"
 #include "pvof_kernels.cuh"
 
 namespace pvof {
@@ -66,7 +66,6 @@ namespace {
 
 constexpr int ROW_THREADS = 256;
 constexpr int ROWG = SPEC_PT / ROW_THREADS;   // row groups per block, one pair of rows each
-constexpr unsigned long long SPEC_SPIN_LIMIT = 1ull << 26;
 constexpr int SPEC_SYS = 8;          // tridiagonal systems per block and pass, one warp each
 constexpr int SPEC_CHUNKS = 32;      // chunks of a system, one per lane
 
@@ -90,81 +89,6 @@ __host__ __device__ inline Chunks spec_chunks(int M)
 // shared-memory column index of row j: one pad double per 32 rows, so the
 // lanes' chunks (about 32 rows apart) fall in different banks
 __device__ __forceinline__ int cidx(int j) { return j + (j >> 5); }
-
-// sum over the block, in a fixed order; the total is valid in thread 0
-__device__ double block_sum(double v, double *sh)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < nw; k++) t += sh[k];
-    return t;
-}
-
-// Grid barrier on a counter of arrivals that the host zeroes before the
-// launch: the launch's g-th barrier is passed once the counter reaches
-// g * gridDim.x (spec_bar_target, kept by the block's thread 0 in shared
-// memory so that it takes no register of the solve; at most four barriers
-// per iteration, so 32 bits hold the count of any iteration cap below
-// about 7 million).  Each block's thread 0 publishes
-// the block's writes (block barrier, device-scope fence), adds its arrival
-// without waiting for the result and polls the counter.  The wait is
-// bounded; returns false (in every thread of the block) when it gave up or
-// another block did.
-__shared__ unsigned spec_bar_target;
-
-__device__ __noinline__ bool spec_barrier(SpecScal *s, int *err)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned target = spec_bar_target += gridDim.x;
-        volatile unsigned *va = &s->arrivals;
-        volatile int *verr = err;
-        int good = 1;
-        __threadfence();
-        atomicAdd(&s->arrivals, 1u);
-        unsigned long long spins = 0;
-        while (*va < target) {
-            ++spins;
-            if ((spins & 1023ull) == 0 && (*verr != 0 || spins > SPEC_SPIN_LIMIT)) {
-                atomicCAS(err, 0, 2);   // 2: the spectral solve's barrier
-                good = 0;
-                break;
-            }
-            if (spins > 4096) __nanosleep(64);
-        }
-        __threadfence();
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
-// this block's sum of v into slot[blockIdx.x]
-__device__ void put_part(double v, double *slot, double *sh)
-{
-    const double b = block_sum(v, sh);
-    if (threadIdx.x == 0) slot[blockIdx.x] = b;
-}
-
-// the sum of a slot over all blocks, in block order, in every thread
-__device__ double slot_total(const double *slot, double *sh)
-{
-    __shared__ double res;
-    double s = 0.0;
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) s += __ldcg(slot + k);
-    const double t = block_sum(s, sh);
-    if (threadIdx.x == 0) res = t;
-    __syncthreads();
-    const double r = res;
-    __syncthreads();
-    return r;
-}
 
 // Complex FFTs of rows of N = R n points (R = 1, 3 or 5, n = 2^logn) by the
 // ROW_THREADS threads of one row group (lt = their index); sign -1 forward.
@@ -495,17 +419,14 @@ __device__ void tridiag_phase(const SpecArgs &A, double *area, bool resident)
 __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, double *d1)
 {
     extern __shared__ double smem[];   // the twiddles, then the row / reduction work area
-    __shared__ double sh[32];
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY, N = A.N, M = A.M;
     const int grp = threadIdx.x / ROW_THREADS, lt = threadIdx.x - grp * ROW_THREADS;
     double2 *tw = reinterpret_cast<double2 *>(smem);
     double *work = smem + N;   // N / 2 complex twiddles before it; the row groups' rows, or the systems' columns
     double2 *row = reinterpret_cast<double2 *>(work) + (size_t)grp * N;
-    double *slotA = A.part, *slotB = A.part + gridDim.x, *slotC = A.part + 2 * gridDim.x;
-    SpecScal *S = A.s;
-    int *err = &A.scal->error;
-    if (threadIdx.x == 0) spec_bar_target = 0;
+    Slots sl{reinterpret_cast<unsigned long long *>(A.part), &A.scal->error, gridDim.x, blockIdx.x, 2, 0};
+    double one[1] = {0.0};   // 2: the spectral solve's exchanges
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     for (int k = threadIdx.x; k < N / 2; k += blockDim.x) tw[k] = A.tw[k];
     __syncthreads();
@@ -531,7 +452,7 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
         stage_tables(A, work + spec_tab_offset(N, M), blockIdx.x * SPEC_SYS);
         cp_async_wait_all();
     }
-    if (!spec_barrier(S, err)) return;
+    if (!grid_exchange<1, true>(sl, one)) return;
 
     // r = rhs - A phi, the stopping sum, forward transforms
     auto residual = [&](int i, int j, double &sum) {
@@ -552,9 +473,9 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
             }
         pair_forward(B, row, ja, acta, actb, lt);
     }
-    put_part(sJ, slotA, sh);
-    if (!spec_barrier(S, err)) return;
-    double tot = slot_total(slotA, sh);
+    one[0] = sJ;
+    if (!grid_exchange<1, true>(sl, one)) return;
+    double tot = one[0];
     int iters = 0;
     double res = sqrt(tot);
     if (sqrt(tot) < A.tol) {   // converged before the first iteration: phi stays as it is
@@ -566,7 +487,8 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
     for (int it = 0;; it++) {
         // z = (-L)^-1 r
         tridiag_phase(A, work, resident);
-        if (!spec_barrier(S, err)) return;
+        one[0] = 0.0;
+        if (!grid_exchange<1, true>(sl, one)) return;
         double g = 0.0;
         for (int p0 = blockIdx.x * ROWG; 2 * p0 < M; p0 += gridDim.x * ROWG) {
             const int ja = 2 * (p0 + grp), jb = ja + 1;
@@ -593,9 +515,9 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
                 }
             __syncthreads();
         }
-        put_part(g, slotB, sh);
-        if (!spec_barrier(S, err)) return;
-        const double gnew = slot_total(slotB, sh);
+        one[0] = g;
+        if (!grid_exchange<1, true>(sl, one)) return;
+        const double gnew = one[0];
         // guards against 0 / 0 only: with the scaling r.z is about the Jacobi
         // weight times smaller than in the reference's iteration, so a guard
         // of the reference's size (1e-30) would bend the steps near a tight
@@ -623,9 +545,9 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
                     sdad += dv * ad;
                 }
             }
-        put_part(sdad, slotC, sh);
-        if (!spec_barrier(S, err)) return;
-        const double alpha = gamma / (slot_total(slotC, sh) + 1e-300);
+        one[0] = sdad;   // the update reads its own rows' d and Ad only
+        if (!grid_exchange<1, false>(sl, one)) return;
+        const double alpha = gamma / (one[0] + 1e-300);
         // phi += alpha d, r -= alpha Ad, the stopping sum, forward transforms
         auto update = [&](int i, int j, double &sum) {
             AT_(A.phi, i, j) += alpha * AT_(dnew, i, j);
@@ -645,9 +567,9 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
                 }
             pair_forward(B, row, ja, acta, actb, lt);
         }
-        put_part(sJ, slotA, sh);
-        if (!spec_barrier(S, err)) return;
-        tot = slot_total(slotA, sh);
+        one[0] = sJ;
+        if (!grid_exchange<1, true>(sl, one)) return;
+        tot = one[0];
         iters = it + 1;
         res = sqrt(tot);
         if (sqrt(tot) < A.tol || iters >= A.maxit) break;
@@ -661,9 +583,9 @@ __global__ void __launch_bounds__(SPEC_PT) k_spec_pcg(SpecArgs A, double *d0, do
             if (j >= M) continue;
             for (int i = lt; i < N; i += ROW_THREADS) ssum += AT_(A.phi, i, j);
         }
-    put_part(ssum, slotB, sh);
-    if (!spec_barrier(S, err)) return;
-    const double avg = slot_total(slotB, sh) / ((double)N * (double)M);
+    one[0] = ssum;
+    if (!grid_exchange<1, false>(sl, one)) return;
+    const double avg = one[0] / ((double)N * (double)M);
     for (int p0 = blockIdx.x * ROWG; 2 * p0 < M; p0 += gridDim.x * ROWG)
         for (int h = 0; h < 2; h++) {
             const int j = 2 * (p0 + grp) + h;
@@ -780,8 +702,8 @@ cudaError_t spec_launch_pcg(const SpecArgs &A, int blocks, double *d0, double *d
 {
     SpecArgs a = A;
     void *args[] = {&a, &d0, &d1};
-    // the grid barriers count arrivals from zero
-    const cudaError_t e = cudaMemsetAsync(&A.s->arrivals, 0, sizeof(unsigned), st);
+    // the exchange slots start from epoch zero
+    const cudaError_t e = cudaMemsetAsync(A.part, 0, spec_slot_doubles(blocks) * sizeof(double), st);
     if (e != cudaSuccess) return e;
     return cudaLaunchCooperativeKernel((const void *)k_spec_pcg, dim3((unsigned)blocks), dim3(SPEC_PT), args,
                                        spec_pcg_smem(A.N, A.M), st);
