@@ -49,10 +49,15 @@ __device__ __forceinline__ void src_of(const BcMap &m, int NX, int NY, int i, in
 // diffuse_solve_biharmonic_pcg (Eulerian/VOF_DIFFUSE.c:339-429): CG on
 // [a_dt I + bih L.L] x = b.  The reference iterates over the G range, whose
 // half cells (i = NX-1, j = NY-1) hold exact copies of their boundary source
-// cells at every iteration; here every physical cell carries the summed
-// measure W of itself and its copies, and both Laplacians of the operator are
-// evaluated on the fly (with the scalar ghost update in between), so one
-// iteration needs two grid barriers.
+// cells at every iteration; here every physical cell carries the summed measure
+// W of itself and its copies.
+// L(p) goes through a field of its own, L of that makes Ap behind a third
+// exchange.  Both Laplacians on the fly would save that exchange and cost five
+// inner Laplacians per cell, 1400 instructions and 140 loads: bound by
+// instruction issue from one cell per thread on.  B200, six solves, on the fly
+// -> two passes: 1024x1024 7.7 -> 4.7 ms, 512x1024 1.24 -> 0.88, 241x482 0.28
+// -> 0.27; below that the exchange costs 0.01 ms (128x512 0.20 -> 0.21), too
+// little for a second form.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
 {
@@ -63,30 +68,30 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double nk = (double)d.nk;
 
-    // L(L(f)) at (i,j) for a field given at sources: lap of the ghost-updated
-    // Laplacian of the ghost-updated f (VOF_DIFFUSE_compute_laplacian twice).
-    auto bilap = [&](int i, int j, auto fsrc) {
-        auto fv = [&](int a, int b) {
+    // L at a physical cell of a field given at physical cells, through the
+    // scalar ghost update (VOF_DIFFUSE_compute_laplacian)
+    auto lap = [&](int i, int j, auto f) {
+        return lap_at(d, i, j, [&](int a, int b) {
             int si, sj;
             double mul;
             src_of(A.msc, NX, NY, a, b, si, sj, mul);
-            return fsrc(si, sj);
-        };
-        auto lapv = [&](int a, int b) {
-            int si, sj;
-            double mul;
-            src_of(A.msc, NX, NY, a, b, si, sj, mul);
-            return lap_at(d, si, sj, fv);
-        };
-        return lap_at(d, i, j, lapv);
+            return f(si, sj);
+        });
     };
+    auto auxf = [&](int a, int b) { return AT_(A.aux, a, b); };
 
+    for (int q = tid; q < R.n; q += nth) {
+        int i, j;
+        R.ij(q, i, j);
+        AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(A.x, a, b); });
+    }
+    double one[1] = {0.0};
+    if (!grid_exchange<1, true>(sl, one)) return;
     double sbb = 0.0, srr = 0.0;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);
-        double l2 = bilap(i, j, [&](int a, int b) { return AT_(A.x, a, b); });
-        double ap = A.a_dt * AT_(A.x, i, j) + A.bih * l2;
+        double ap = A.a_dt * AT_(A.x, i, j) + A.bih * lap(i, j, auxf);
         double bv = AT_(A.b, i, j);
         double rv = bv - ap;
         AT_(A.r, i, j) = rv;
@@ -95,7 +100,7 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
         sbb += m * bv * bv;
         srr += m * rv * rv;
     }
-    double both[2] = {sbb, srr}, one[1];
+    double both[2] = {sbb, srr};
     if (!grid_exchange<2, true>(sl, both)) return;
     double rhs_norm = sqrt(nk * both[0]);
     if (rhs_norm < 1e-30) rhs_norm = 1.0;
@@ -117,23 +122,27 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
         for (int q = tid; q < R.n; q += nth) {
             int i, j;
             R.ij(q, i, j);
-            double pv, l2;
             if (first) {
-                pv = AT_(pold, i, j);
-                l2 = bilap(i, j, [&](int a, int b) { return AT_(pold, a, b); });
+                AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(pold, a, b); });
             } else {
                 const double po = AT_(pold, i, j);
-                pv = AT_(A.r, i, j) + bt * po;
-                AT_(pnxt, i, j) = pv;
+                AT_(pnxt, i, j) = AT_(A.r, i, j) + bt * po;
                 AT_(A.x, i, j) += al * po;   // the update of the iteration before
-                l2 = bilap(i, j, [&](int a, int b) { return AT_(A.r, a, b) + bt * AT_(pold, a, b); });
+                AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(A.r, a, b) + bt * AT_(pold, a, b); });
             }
-            double ap = A.a_dt * pv + A.bih * l2;
-            AT_(A.Ap, i, j) = ap;
-            spap += d.m.wx[i] * d.m.wy[j] * d.wz * pv * ap;
         }
         if (!first) { double *t = pcur; pcur = pnxt; pnxt = t; }
         first = false;
+        one[0] = 0.0;
+        if (!grid_exchange<1, true>(sl, one)) return;
+        for (int q = tid; q < R.n; q += nth) {
+            int i, j;
+            R.ij(q, i, j);
+            const double pv = AT_(pcur, i, j);
+            const double ap = A.a_dt * pv + A.bih * lap(i, j, auxf);
+            AT_(A.Ap, i, j) = ap;
+            spap += d.m.wx[i] * d.m.wy[j] * d.wz * pv * ap;
+        }
         // the update reads its own cells' Ap only: the sum alone
         one[0] = spap;
         pending = false;
