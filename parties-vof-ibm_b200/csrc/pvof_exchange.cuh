@@ -23,6 +23,9 @@ constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;   // polls of one 
 // epoch, so a word is valid by itself and the two need not arrive together.
 // Two buffers alternate: a block writes epoch e + 2 only after it has the
 // totals of e + 1, which need every block's e + 1, published after it read e.
+// Both begin at the same place whatever NV is (slots are NV doubles apart
+// inside), so an exchange of two sums right behind one of one sum does not
+// write over slots that are still read.
 // The host zeroes the slots before each launch; epochs start at 1.  The sums
 // are taken in a fixed order (a tree in the block, then the blocks by lane), so
 // every block has the same totals and runs repeat bit for bit.
@@ -32,7 +35,7 @@ constexpr unsigned long long BARRIER_SPIN_LIMIT = 1ull << 26;   // polls of one 
 // a fence in the first block before the totals.  False, in every thread of the block,
 // when the bounded wait gave up.
 struct Slots {
-    unsigned long long *w;   // two buffers of nb + 1 slots
+    unsigned long long *w;   // two buffers of nb + 1 slots of up to SLOT_SUMS sums
     int *error;
     unsigned nb, rank;       // blocks that exchange with one another, this block's number among them
     int code;                // what DevScalars::error says when a wait gives up
@@ -93,7 +96,8 @@ __device__ __forceinline__ bool grid_exchange(Slots &sl, double (&v)[NV])
     auto &total = S.total;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const unsigned nb = sl.nb, rank = sl.rank, e = ++sl.epoch;
-    unsigned long long *buf = sl.w + (size_t)(e & 1u) * (nb + 1) * 2 * NV;
+    static_assert(NV <= SLOT_SUMS, "a slot buffer holds SLOT_SUMS sums per block");
+    unsigned long long *buf = sl.w + (size_t)(e & 1u) * (nb + 1) * 2 * SLOT_SUMS;
     int good = 1;
 #pragma unroll
     for (int n = 0; n < NV; n++)

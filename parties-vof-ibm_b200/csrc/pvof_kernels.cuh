@@ -39,7 +39,8 @@ struct VelArgs {
 
 // doubles per block (and one more) of the grid-wide solvers' exchange slots: two
 // buffers of two values, two words per value
-constexpr size_t SLOT_DOUBLES = 8;
+constexpr int SLOT_SUMS = 2;   // most sums of one exchange
+constexpr size_t SLOT_DOUBLES = 2 * 2 * SLOT_SUMS;
 constexpr int SLOT_BLOCKS = 320;   // most blocks of an exchange (two per SM of a B200 are 296)
 
 struct PresArgs {
@@ -57,7 +58,7 @@ struct PresArgs {
 
 // spectral-preconditioned pressure PCG (pvof_spec.cu)
 constexpr int SPEC_PT = 1024;        // threads per block of the cooperative solve
-constexpr size_t spec_slot_doubles(int blocks) { return 4 * ((size_t)blocks + 1); }
+constexpr size_t spec_slot_doubles(int blocks) { return SLOT_DOUBLES * ((size_t)blocks + 1); }
 
 struct SpecArgs {
     Dom d;
