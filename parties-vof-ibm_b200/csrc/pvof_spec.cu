@@ -684,9 +684,8 @@ size_t spec_pcg_smem(int N, int M)
 int spec_pcg_blocks(int device, int N, int M)
 {
     const size_t smem = spec_pcg_smem(N, M);
-    if (smem > 48 * 1024 &&
-        !raise_dynamic_smem((const void *)k_spec_pcg, smem))
-        return 0;
+    // the default limit of 48 KB covers static and dynamic shared memory together
+    if (!raise_dynamic_smem((const void *)k_spec_pcg, smem)) return 0;
     int per_sm = 0, sms = 0, coop = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spec_pcg, SPEC_PT, smem) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return 0;
