@@ -39,6 +39,7 @@
 // u and v momentum iteration 9.1 -> 5.4 us (whose weights are kept inverted
 // too, no division left in it).  The per-cell arithmetic is otherwise the
 // reference's: the same operands in the same order.
+#include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdlib>
 #include <mutex>
@@ -839,6 +840,41 @@ static bool identity_on(const std::vector<int> &src, const std::vector<double> &
     return true;
 }
 
+// Cells per thread of the form that runs a W x H range: the loops have no
+// branches, so a thread pays for CPT cells however few its strip has.  512
+// threads: the smallest of 2, 4 and 8 that holds the longest strip.  B200, one
+// step, 8 cells for every range -> this rule: 32x64 3.73 -> 2.74 ms, 64x160
+// axisymmetric 8.47 -> 5.66, 100x200 7.36 -> 5.67; 128x512 needs the 8.
+static int strip_cells(int W, int H, int NT)
+{
+    if (NT == 1024) return 4;
+    const int NRmax = (H + CGC_CTAS - 1) / CGC_CTAS, nband = NT / W, nr = (NRmax + nband - 1) / nband;
+    return nr <= 2 ? 2 : (nr <= 4 ? 4 : 8);
+}
+
+template <bool AXI>
+static void (*pressure_kernel(int NT, int cpt))(PresArgs)
+{
+    if (NT == 1024) return k_cgs_pressure<1024, 4, AXI>;
+    return cpt == 2 ? k_cgs_pressure<512, 2, AXI> : (cpt == 4 ? k_cgs_pressure<512, 4, AXI> : k_cgs_pressure<512, 8, AXI>);
+}
+static void (*pressure_kernel(int W, int H, int NT, bool axi))(PresArgs)
+{
+    const int cpt = strip_cells(W, H, NT);
+    return axi ? pressure_kernel<true>(NT, cpt) : pressure_kernel<false>(NT, cpt);
+}
+
+template <bool AXI>
+static void (*velocity_kernel(int NT, int cpt))(VelPair)
+{
+    if (NT == 1024) return k_cgs_velocity<1024, 4, AXI>;
+    return cpt == 2 ? k_cgs_velocity<512, 2, AXI> : (cpt == 4 ? k_cgs_velocity<512, 4, AXI> : k_cgs_velocity<512, 8, AXI>);
+}
+static void (*velocity_kernel(int cpt, int NT, bool axi))(VelPair)
+{
+    return axi ? velocity_kernel<true>(NT, cpt) : velocity_kernel<false>(NT, cpt);
+}
+
 StripPlan cgs_pressure_setup(int NX, int NY, int axisym, const HostMap &mp)
 {
     StripPlan plan = {0, 0};
@@ -847,14 +883,10 @@ StripPlan cgs_pressure_setup(int NX, int NY, int axisym, const HostMap &mp)
     if (!strip_edges_ok(mp.ysrc, mp.ymul, 0, H)) return plan;
     size_t smem;
     // 512 threads first: the 1024-thread form spills at 64 registers per thread
-    if ((smem = strip_smem(W, H, 0, 512, 8)) &&
-        (axisym ? strip_kernel_fits(k_cgs_pressure<512, 8, true>, 512, smem)
-                : strip_kernel_fits(k_cgs_pressure<512, 8, false>, 512, smem)))
-        return StripPlan{smem, 512};
-    if ((smem = strip_smem(W, H, 0, 1024, 4)) &&
-        (axisym ? strip_kernel_fits(k_cgs_pressure<1024, 4, true>, 1024, smem)
-                : strip_kernel_fits(k_cgs_pressure<1024, 4, false>, 1024, smem)))
-        return StripPlan{smem, 1024};
+    for (int nt : {512, 1024})
+        if ((smem = strip_smem(W, H, 0, nt, nt == 1024 ? 4 : 8)) &&
+            strip_kernel_fits(pressure_kernel(W, H, nt, axisym != 0), nt, smem))
+            return StripPlan{smem, nt};
     return plan;
 }
 
@@ -862,12 +894,7 @@ cudaError_t cgs_pressure_launch(const PresArgs &A, const StripPlan &plan, cudaSt
 {
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = strip_config(1, plan.threads, plan.smem, stream, at);
-    const bool axi = A.d.axisym != 0;
-    if (plan.threads == 1024)
-        return axi ? cudaLaunchKernelEx(&cfg, k_cgs_pressure<1024, 4, true>, A)
-                   : cudaLaunchKernelEx(&cfg, k_cgs_pressure<1024, 4, false>, A);
-    return axi ? cudaLaunchKernelEx(&cfg, k_cgs_pressure<512, 8, true>, A)
-               : cudaLaunchKernelEx(&cfg, k_cgs_pressure<512, 8, false>, A);
+    return cudaLaunchKernelEx(&cfg, pressure_kernel(A.d.NX - 1, A.d.NY - 1, plan.threads, A.d.axisym != 0), A);
 }
 
 static bool velocity_range_ok(const int r[4], const HostMap &mcg)
@@ -888,12 +915,11 @@ StripPlan cgs_velocity_setup(const int ru[4], const HostMap &mu, const int rv[4]
         const size_t su = strip_smem(Wu, Hu, 1, nt, cpt), sv = strip_smem(Wv, Hv, 1, nt, cpt);
         if (!su || !sv) continue;
         const size_t smem = su > sv ? su : sv;
-        bool ok;
-        if (nt == 1024) ok = axisym ? strip_kernel_fits(k_cgs_velocity<1024, 4, true>, nt, smem)
-                                    : strip_kernel_fits(k_cgs_velocity<1024, 4, false>, nt, smem);
-        else ok = axisym ? strip_kernel_fits(k_cgs_velocity<512, 8, true>, nt, smem)
-                         : strip_kernel_fits(k_cgs_velocity<512, 8, false>, nt, smem);
-        if (ok) return StripPlan{smem, nt};
+        // u and v together and either alone (one component per launch)
+        const int cu = strip_cells(Wu, Hu, nt), cv = strip_cells(Wv, Hv, nt);
+        if (strip_kernel_fits(velocity_kernel(cu, nt, axisym != 0), nt, smem) &&
+            strip_kernel_fits(velocity_kernel(cv, nt, axisym != 0), nt, smem))
+            return StripPlan{smem, nt};
     }
     return plan;
 }
@@ -902,12 +928,10 @@ cudaError_t cgs_velocity_launch(const VelPair &V, int ncomp, const StripPlan &pl
 {
     cudaLaunchAttribute at[1];
     cudaLaunchConfig_t cfg = strip_config(ncomp, plan.threads, plan.smem, stream, at);
-    const bool axi = V.c[0].d.axisym != 0;
-    if (plan.threads == 1024)
-        return axi ? cudaLaunchKernelEx(&cfg, k_cgs_velocity<1024, 4, true>, V)
-                   : cudaLaunchKernelEx(&cfg, k_cgs_velocity<1024, 4, false>, V);
-    return axi ? cudaLaunchKernelEx(&cfg, k_cgs_velocity<512, 8, true>, V)
-               : cudaLaunchKernelEx(&cfg, k_cgs_velocity<512, 8, false>, V);
+    int cpt = 0;
+    for (int q = 0; q < ncomp; q++)
+        cpt = std::max(cpt, strip_cells(V.c[q].i1 - V.c[q].i0, V.c[q].j1 - V.c[q].j0, plan.threads));
+    return cudaLaunchKernelEx(&cfg, velocity_kernel(cpt, plan.threads, V.c[0].d.axisym != 0), V);
 }
 
 }  // namespace pvof
