@@ -8,13 +8,13 @@
 // grid-stride mapping in every phase, so a thread reads back its own cells'
 // private values (diagonal, Ad) without a barrier.
 //
-// Two grid barriers per iteration: the new search direction d_k = z_k +
-// beta d_{k-1} is not written in a phase of its own; the matrix-vector phase
-// writes it for its own cells into the second direction buffer and evaluates
-// it on the fly at the stencil neighbours (from z and d_{k-1}, with the
-// reference's ghost update of d applied through the same source maps).  The
-// arithmetic per value is the reference's, so the iterates are those of the
-// reference's loop.
+// Two grid barriers per iteration (three in the biharmonic solve): the new
+// search direction d_k = z_k + beta d_{k-1} is not written in a phase of its
+// own; the matrix-vector phase writes it for its own cells into the second
+// direction buffer and evaluates it on the fly at the stencil neighbours (from
+// z and d_{k-1}, with the reference's ghost update of d applied through the
+// same source maps).  The arithmetic per value is the reference's, so the
+// iterates are those of the reference's loop.
 //
 // The grid barriers are this file's own (not cooperative_groups::grid_group::
 // sync) so that their waits are bounded: if the other blocks never arrive
