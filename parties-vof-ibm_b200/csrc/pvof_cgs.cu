@@ -115,25 +115,36 @@ struct EdgePair {
     int dst[2][2];           // their rank * 2 + side
 };
 
-// Fills `ep` (thread 0) for the rows below and above the slab that starts at
-// range row j0 of the ghost map's index space rj0.
+// Fills `ep` for the rows below and above the slab that starts at range row j0
+// of the ghost map's index space rj0: by one warp, a lane per slab and side (a
+// solve of few iterations feels a serial walk of all slabs: B200, momentum
+// solve of u and v with four iterations at 64x300: one thread 51 us, a warp
+// 27).
 __device__ inline void edge_pair(EdgePair &ep, const AxisMap &ym, int rj0, int H, int nb, int rank, int *error)
 {
-    ep.ndst[0] = ep.ndst[1] = 0;
-    for (int c = 0; c < nb; c++)
-        for (int q = 0; q < 2; q++) {
-            const int b = q ? slab_row0(c + 1, H, nb) : slab_row0(c, H, nb) - 1;
-            const SlabEdge e = slab_edge(ym.src, ym.mul, rj0, H, nb, c, rj0 + b, error);
-            if (c == rank) {
-                ep.mul[q] = e.mul;
-                ep.local[q] = e.local;
-                ep.lrow[q] = e.lrow;
-            }
-            if (!e.local && e.owner == rank) {
-                if (ep.ndst[e.zsel] < 2) ep.dst[e.zsel][ep.ndst[e.zsel]++] = 2 * c + q;
-                else atomicCAS(error, 0, 3);   // a row has at most two readers: the slab beyond it and a periodic image
-            }
+    const int lane = threadIdx.x & 31, c = lane >> 1, q = lane & 1;
+    static_assert(2 * CGC_CTAS <= 32, "a lane per slab and side");
+    SlabEdge e = {0.0, 1, 0, 0, -1};
+    if (c < nb) {
+        const int b = q ? slab_row0(c + 1, H, nb) : slab_row0(c, H, nb) - 1;
+        e = slab_edge(ym.src, ym.mul, rj0, H, nb, c, rj0 + b, error);
+        if (c == rank) {
+            ep.mul[q] = e.mul;
+            ep.local[q] = e.local;
+            ep.lrow[q] = e.lrow;
         }
+    }
+#pragma unroll
+    for (int z = 0; z < 2; z++) {
+        const bool reads = !e.local && e.owner == rank && e.zsel == z;   // this lane's slab reads our row z
+        const unsigned m = __ballot_sync(0xffffffffu, reads);
+        const int at = __popc(m & ((1u << lane) - 1u));
+        if (reads && at < 2) ep.dst[z][at] = 2 * c + q;
+        if (lane == 0) {
+            ep.ndst[z] = min(__popc(m), 2);
+            if (__popc(m) > 2) atomicCAS(error, 0, 3);   // a row has at most two readers: the slab beyond it and a periodic image
+        }
+    }
 }
 
 // Column source of the east/west neighbour a (range coordinates) of a thread.
@@ -340,10 +351,8 @@ __global__ void __launch_bounds__(NT, 1) k_cgs_pressure(PresArgs A)
     __shared__ EdgePair ep;
     __shared__ GhostCols gcs;
 
-    if (threadIdx.x == 0) {
-        edge_pair(ep, A.mp.y, 0, H, s.nb, s.rank, &A.scal->error);
-        gcs = ghost_cols(A.mp.x, 0, W);
-    }
+    if (threadIdx.x < 32) edge_pair(ep, A.mp.y, 0, H, s.nb, s.rank, &A.scal->error);
+    if (threadIdx.x == 32) gcs = ghost_cols(A.mp.x, 0, W);
     for (int q = threadIdx.x; q < NRmax * Wp; q += NT) pb[q] = 0.0;   // zero ghosts
     inbox_init(cl, ib);
     const int rows = ((!ep.local[0] ? 1 : 0) + (!ep.local[1] ? 1 : 0)) * W;
@@ -583,10 +592,8 @@ __global__ void __launch_bounds__(NT, 1) k_cgs_velocity(const __grid_constant__ 
         if (AXI) { rce = d.m.r_u[i + 1]; rcw = d.m.r_u[i]; iru = d.m.inv_r_c[i]; }
     }
 
-    if (threadIdx.x == 0) {
-        edge_pair(ep, A.mcg.y, A.j0, H, nb, s.rank, &A.scal->error);
-        gcs = ghost_cols(A.mcg.x, A.i0, W);
-    }
+    if (threadIdx.x < 32) edge_pair(ep, A.mcg.y, A.j0, H, nb, s.rank, &A.scal->error);
+    if (threadIdx.x == 32) gcs = ghost_cols(A.mcg.x, A.i0, W);
     for (int q = threadIdx.x; q < NRmax * Wp; q += NT) pb[q] = 0.0;   // zero ghosts
     inbox_init(cl, ib);
     const int rows = ((!ep.local[0] ? 1 : 0) + (!ep.local[1] ? 1 : 0)) * W;
