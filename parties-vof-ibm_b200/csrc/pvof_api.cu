@@ -412,10 +412,11 @@ int timed_launch(pvof_ctx *c, int kind, int comp, int n, L launch, int n2 = 0)
     return PVOF_OK;
 }
 
+// most: co-resident blocks of fn, where fewer than its solver's other kernels take
 template <class A>
-int coop_launch(pvof_ctx *c, const void *fn, A &args, int n, int kind, int comp)
+int coop_launch(pvof_ctx *c, const void *fn, A &args, int n, int kind, int comp, int most = SLOT_BLOCKS)
 {
-    int nb = coop_blocks(c, n, kind);
+    const int nb = std::min(coop_blocks(c, n, kind), most);
     // the solvers' exchange slots start from epoch zero
     CK(cudaMemsetAsync(c->partials, 0, SLOT_DOUBLES * (size_t)(nb + 1) * sizeof(double), c->stream));
     return timed_launch(c, kind, comp, n, [&]() {
@@ -549,6 +550,18 @@ int vof_diffuse_init(pvof_ctx *c)
     return fill(c, BK_SCALAR, F(c, PVOF_F_C_G));
 }
 
+// The biharmonic solve evaluates both Laplacians on the fly (two exchanges an
+// iteration) as long as one block per SM holds the range at a cell per thread:
+// its registers allow one block per SM, and a second cell per thread, or two
+// blocks at 64 registers, cost more than the third exchange of the form through a
+// field.  B200, us a solve, on the fly | field: 32x64 28.5 | 28.9, 64x300 38.0 |
+// 44.4, 128x512 40.0 | 44.9, 256x256 67.3 | 78.5, 296x256 (75 776 cells, the last)
+// 91 | 100, 300x256 115 | 103, 512x512 (64 registers) 527 | 399.
+bool biharmonic_on_the_fly(const pvof_ctx *c)
+{
+    return (c->dom.NX - 1) * (c->dom.NY - 1) <= c->bih_fly_blocks * COOP_THREADS;
+}
+
 int vof_diffuse_step(pvof_ctx *c)
 {
     const int NX = c->dom.NX, NY = c->dom.NY, s = c->stage;
@@ -589,7 +602,9 @@ int vof_diffuse_step(pvof_ctx *c)
     A.maxit = (c->p.ch_iter_max > 0) ? c->p.ch_iter_max : c->p.CG_MAXIT;
     A.partials = c->partials;
     A.scal = c->scal;
-    TRY(coop_launch(c, (const void *)k_cg_biharmonic, A, NX * NY, PVOF_SOLVER_BIHARMONIC, 0));
+    if (biharmonic_on_the_fly(c))
+        TRY(coop_launch(c, (const void *)k_cg_biharmonic_fly, A, NX * NY, PVOF_SOLVER_BIHARMONIC, 0, c->bih_fly_blocks));
+    else TRY(coop_launch(c, (const void *)k_cg_biharmonic, A, NX * NY, PVOF_SOLVER_BIHARMONIC, 0));
     TRY(fill(c, BK_SCALAR, CL));
     // clamp, phase cache, history shift (VOF_DIFFUSE.c:1324-1358)
     TRY(bound(c));
@@ -1161,7 +1176,8 @@ bool keep_cooperative(cudaGraph_t g)
     if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess) return false;
     std::vector<cudaGraphNode_t> nodes(n);
     if (n && cudaGraphGetNodes(g, nodes.data(), &n) != cudaSuccess) return false;
-    const void *coop[] = {(const void *)k_cg_biharmonic, (const void *)k_cg_velocity, (const void *)k_cg_velocity_res,
+    const void *coop[] = {(const void *)k_cg_biharmonic, (const void *)k_cg_biharmonic_fly, (const void *)k_cg_velocity,
+                          (const void *)k_cg_velocity_res,
                           (const void *)k_cg_pressure_fw,
                           (const void *)k_cg_pressure_fwp,
                           spec_pcg_kernel()};
@@ -1938,6 +1954,11 @@ int pvof_create(const pvof_grid_desc *grid, const pvof_params *params, int devic
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     if (!coop) return fail(PVOF_ENODEV, "device without cooperative launch");
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_cg_biharmonic, COOP_THREADS, 0);
+    {
+        int o1f = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1f, k_cg_biharmonic_fly, COOP_THREADS, 0);
+        c->bih_fly_blocks = std::min(o1f * nsm, SLOT_BLOCKS);
+    }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_cg_velocity, COOP_THREADS, 0);
     {   // the two grid-wide velocity kernels take the same block count
         int o2r = 0;
@@ -2459,7 +2480,7 @@ const char *pvof_solver_kernel(const pvof_ctx *c, int solver)
         return (solver >= 0 && solver <= 2) ? k3[solver] : "";
     }
     switch (solver) {
-    case PVOF_SOLVER_BIHARMONIC: return "k_cg_biharmonic";
+    case PVOF_SOLVER_BIHARMONIC: return biharmonic_on_the_fly(c) ? "k_cg_biharmonic_fly" : "k_cg_biharmonic";
     case PVOF_SOLVER_VELOCITY: {
         if (c->cgs_v_smem) return "k_cgs_velocity";
         int n[2], i0, i1, j0, j1;

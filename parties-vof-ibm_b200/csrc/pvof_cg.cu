@@ -51,15 +51,16 @@ __device__ __forceinline__ void src_of(const BcMap &m, int NX, int NY, int i, in
 // half cells (i = NX-1, j = NY-1) hold exact copies of their boundary source
 // cells at every iteration; here every physical cell carries the summed measure
 // W of itself and its copies.
-// L(p) goes through a field of its own, L of that makes Ap behind a third
-// exchange.  Both Laplacians on the fly would save that exchange and cost five
-// inner Laplacians per cell, 1400 instructions and 140 loads: bound by
-// instruction issue from one cell per thread on.  B200, six solves, on the fly
-// -> two passes: 1024x1024 7.7 -> 4.7 ms, 512x1024 1.24 -> 0.88, 241x482 0.28
-// -> 0.27; below that the exchange costs 0.01 ms (128x512 0.20 -> 0.21), too
-// little for a second form.
+// Two forms of L(L(p)), the same operands in the same operations.  FLY: both
+// Laplacians on the fly, two exchanges an iteration, five inner Laplacians per
+// cell (1400 instructions, 140 loads).  Otherwise L(p) goes through a field of its
+// own and L of that makes Ap behind a third exchange.  The context picks by the
+// number of cells (biharmonic_on_the_fly).  Bound by the latency of the exchanges
+// on small ranges, by L2 from about 300 000 cells on: 1024x1024, six solves, on
+// the fly 7.7 ms, through the field 4.7.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
+template <bool FLY>
+__device__ __forceinline__ void cg_biharmonic(const BihArgs &A)
 {
     const Dom &d = A.d;
     const int P = d.P, NX = d.NX, NY = d.NY;
@@ -68,8 +69,8 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     const double nk = (double)d.nk;
 
-    // L at a physical cell of a field given at physical cells, through the
-    // scalar ghost update (VOF_DIFFUSE_compute_laplacian)
+    // L at a cell of a field given at physical cells, through the scalar ghost
+    // update (VOF_DIFFUSE_compute_laplacian)
     auto lap = [&](int i, int j, auto f) {
         return lap_at(d, i, j, [&](int a, int b) {
             int si, sj;
@@ -79,19 +80,24 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
         });
     };
     auto auxf = [&](int a, int b) { return AT_(A.aux, a, b); };
+    // L(L(f)) without and with the field
+    auto twice = [&](int i, int j, auto f) { return lap(i, j, [&](int a, int b) { return lap(a, b, f); }); };
 
-    for (int q = tid; q < R.n; q += nth) {
-        int i, j;
-        R.ij(q, i, j);
-        AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(A.x, a, b); });
-    }
     double one[1] = {0.0};
-    if (!grid_exchange<1, true>(sl, one)) return;
+    auto xf = [&](int a, int b) { return AT_(A.x, a, b); };
+    if (!FLY) {
+        for (int q = tid; q < R.n; q += nth) {
+            int i, j;
+            R.ij(q, i, j);
+            AT_(A.aux, i, j) = lap(i, j, xf);
+        }
+        if (!grid_exchange<1, true>(sl, one)) return;
+    }
     double sbb = 0.0, srr = 0.0;
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);
-        double ap = A.a_dt * AT_(A.x, i, j) + A.bih * lap(i, j, auxf);
+        double ap = A.a_dt * AT_(A.x, i, j) + A.bih * (FLY ? twice(i, j, xf) : lap(i, j, auxf));
         double bv = AT_(A.b, i, j);
         double rv = bv - ap;
         AT_(A.r, i, j) = rv;
@@ -122,26 +128,39 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
         for (int q = tid; q < R.n; q += nth) {
             int i, j;
             R.ij(q, i, j);
+            const double po = AT_(pold, i, j);
+            double pv = po, l;
             if (first) {
-                AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(pold, a, b); });
+                auto p = [&](int a, int b) { return AT_(pold, a, b); };
+                l = FLY ? twice(i, j, p) : lap(i, j, p);
             } else {
-                const double po = AT_(pold, i, j);
-                AT_(pnxt, i, j) = AT_(A.r, i, j) + bt * po;
+                pv = AT_(A.r, i, j) + bt * po;
+                AT_(pnxt, i, j) = pv;
                 AT_(A.x, i, j) += al * po;   // the update of the iteration before
-                AT_(A.aux, i, j) = lap(i, j, [&](int a, int b) { return AT_(A.r, a, b) + bt * AT_(pold, a, b); });
+                auto p = [&](int a, int b) { return AT_(A.r, a, b) + bt * AT_(pold, a, b); };
+                l = FLY ? twice(i, j, p) : lap(i, j, p);
+            }
+            if (FLY) {
+                const double ap = A.a_dt * pv + A.bih * l;
+                AT_(A.Ap, i, j) = ap;
+                spap += d.m.wx[i] * d.m.wy[j] * d.wz * pv * ap;
+            } else {
+                AT_(A.aux, i, j) = l;
             }
         }
         if (!first) { double *t = pcur; pcur = pnxt; pnxt = t; }
         first = false;
-        one[0] = 0.0;
-        if (!grid_exchange<1, true>(sl, one)) return;
-        for (int q = tid; q < R.n; q += nth) {
-            int i, j;
-            R.ij(q, i, j);
-            const double pv = AT_(pcur, i, j);
-            const double ap = A.a_dt * pv + A.bih * lap(i, j, auxf);
-            AT_(A.Ap, i, j) = ap;
-            spap += d.m.wx[i] * d.m.wy[j] * d.wz * pv * ap;
+        if (!FLY) {
+            one[0] = 0.0;
+            if (!grid_exchange<1, true>(sl, one)) return;
+            for (int q = tid; q < R.n; q += nth) {
+                int i, j;
+                R.ij(q, i, j);
+                const double pv = AT_(pcur, i, j);
+                const double ap = A.a_dt * pv + A.bih * lap(i, j, auxf);
+                AT_(A.Ap, i, j) = ap;
+                spap += d.m.wx[i] * d.m.wy[j] * d.wz * pv * ap;
+            }
         }
         // the update reads its own cells' Ap only: the sum alone
         one[0] = spap;
@@ -189,6 +208,10 @@ __global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A)
         }
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->ch_iters = iter; A.scal->ch_rel = rel; }
 }
+
+__global__ void __launch_bounds__(512, 2) k_cg_biharmonic(BihArgs A) { cg_biharmonic<false>(A); }
+// one block per SM: at 64 registers (two) it spills, 256x256 75.0 us against 70.9
+__global__ void __launch_bounds__(512) k_cg_biharmonic_fly(BihArgs A) { cg_biharmonic<true>(A); }
 
 // ---------------------------------------------------------------------------
 // One cell per thread: every value of the solve that belongs to the cell stays

@@ -172,6 +172,7 @@ struct Ctx {
     float *cnn_x, *cnn_y, *cnn_work;
     int coop_blocks;         // the most co-resident blocks of any grid-wide solver (sizes the partial sums)
     int coop_blocks_of[3];   // co-resident blocks of each grid-wide solver, by PVOF_SOLVER_*
+    int bih_fly_blocks;      // co-resident blocks of the biharmonic solve's on-the-fly form
     int coop_threads;
     long long launches;      // kernels launched by this context
     // measurement

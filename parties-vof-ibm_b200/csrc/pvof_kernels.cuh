@@ -281,6 +281,7 @@ cudaError_t fft_solve_launch(const Dom &d, const FftArgs &A, const double *thoma
                              double *out, cudaStream_t st);
 
 __global__ void k_cg_biharmonic(BihArgs A);
+__global__ void k_cg_biharmonic_fly(BihArgs A);
 __global__ void k_cg_velocity(VelArgs A);
 __global__ void k_cg_velocity_res(VelArgs A);
 __global__ void k_cg_pressure(PresArgs A);
