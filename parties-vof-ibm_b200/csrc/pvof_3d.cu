@@ -116,24 +116,49 @@ __global__ void __launch_bounds__(TPB) k3_scalar(const double *part, Pend pd, co
 }
 
 // ---------------------------------------------------------------------------
-// the pressure PCG iteration (psolve_cg.c:209-253) as two streaming kernels
+// the pressure PCG iteration (psolve_cg.c:209-253) as three streaming kernels
 // over the physical cells: a thread takes two neighbouring cells of a row
 // (16-byte loads; i = 0 is 16-byte aligned and every row and plane pitch is
-// even) in PKB or PKD consecutive planes, a block a 64 x 8 tile of (i, j);
-// several planes per block keep the end-of-block reduction barrier and the number of
-// partial sums small.  The arithmetic is that of p_apply_st and of the
-// reference's loops, operand for operand.
+// even) in PKB consecutive planes, a block a 64 x 8 tile of (i, j); PKB
+// planes per block keep the end-of-block reduction barrier and the number of
+// partial sums small.  Reads at
+// ghost and half cells go through the pressure ghost map; the arithmetic is
+// that of p_apply_st and of the reference's loops, operand for operand.
+// Bound by HBM from about 2 million cells on (256^3: 13 fields, 395 us), below by
+// latency and launches.  Three passes: one that forms the direction, applies the
+// operator and updates phi together moves nine fields, but its three planes in
+// registers leave three blocks per SM, whose last wave is mostly empty just
+// above 444 blocks.  Us an iteration, three passes | two: 64^3 24.6 | 27.6, 96^3
+// 34.5 | 33.9, 120x97x104 42 | 43, 120^3 57.3 | 72.1, 128^3 66 | 81, 160^3 124 |
+// 128, 256x128x64 64 | 79, 256^3 395 | 407.
 // ---------------------------------------------------------------------------
-constexpr int PKB = 4;   // of the passes without a stencil and of the momentum passes
-constexpr int PKD = 8;   // of the pressure direction pass, which starts a block with two more planes (120x97x104 28.9 us with 4, 26.1 with 8)
+constexpr int PKB = 4;   // the momentum passes' too
 
 __device__ __forceinline__ double2 ld2(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 __device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
 
+// the cells (i, i+1) of a pressure field at (j, k), after the ghost update
+__device__ __forceinline__ void p_pair(const Dom3 &d, const double *__restrict__ X, int i, int j, int k, double &a,
+                                       double &b)
+{
+    if (j >= 0 && j <= d.NY - 2 && k >= 0 && k <= d.NZ - 2) {
+        const double2 v = ld2(X + at(d, i, j, k));
+        a = v.x;
+        b = v.y;
+    } else {
+        a = rd<K_PRESSURE>(d, X, i, j, k);
+        b = rd<K_PRESSURE>(d, X, i + 1, j, k);
+    }
+}
+
 // The sums of a block of 256 threads into part[block]; the last block to finish
 // adds all the partials in a fixed order (the same whichever block is last) and
 // runs the scalar step then(sc, sums...) on one thread, so no separate launch
-// is needed between the passes.
+// is needed between the passes.  The last block's loads go out eight at a time, at
+// the last partial again instead of tested beyond it (with a test each the
+// pressure iteration took 405 us at 256^3 against 395, 82.5 at 127^3 against 80.3;
+// one by one behind the last full eight, the momentum iteration 101.6 at 120^3
+// against 98.7).
 template <int NV, class F>
 __device__ __forceinline__ void block_sum_then(double (&acc)[NV], double *part, Sc3 *sc, F then)
 {
@@ -166,16 +191,16 @@ __device__ __forceinline__ void block_sum_then(double (&acc)[NV], double *part, 
     __threadfence();
 #pragma unroll
     for (int n = 0; n < NV; n++) acc[n] = 0.0;
-    for (unsigned b = t; b < nb; b += 8 * 256) {   // eight loads in flight per thread
+    for (unsigned b = t; b < nb; b += 8 * 256) {   // beyond the last partial: that one again, not added
         double v[8][NV];
 #pragma unroll
         for (int u = 0; u < 8; u++)
 #pragma unroll
-            for (int n = 0; n < NV; n++) v[u][n] = b + u * 256 < nb ? __ldcg(part + (size_t)(b + u * 256) * 4 + n) : 0.0;
+            for (int n = 0; n < NV; n++) v[u][n] = __ldcg(part + (size_t)min(b + u * 256, nb - 1) * 4 + n);
 #pragma unroll
         for (int u = 0; u < 8; u++)
 #pragma unroll
-            for (int n = 0; n < NV; n++) acc[n] += v[u][n];
+            for (int n = 0; n < NV; n++) acc[n] += b + u * 256 < nb ? v[u][n] : 0.0;
     }
     __syncthreads();
     block_sum();
@@ -186,113 +211,60 @@ __device__ __forceinline__ void block_sum_then(double (&acc)[NV], double *part, 
     }
 }
 
-// First pass: phi += alpha d_old of the iteration before, the direction d = z +
-// beta d_old, A d and d.Ad.  A thread marches PKD planes in z with the
-// directions of three planes in registers; its east and west neighbours come
-// from the neighbouring lanes, north and south from the tile in shared memory,
-// and only the tile's edges form a neighbour's direction themselves (the
-// neighbour's operands and operation).  One pass where forming d, applying the
-// operator and updating phi were three: nine fields moved instead of thirteen
-// and a launch less.  Bound by HBM from about 2 million cells on (256^3 290 us
-// against 199 + about 90 of the update's 151 for its parts); below, by latency
-// and launches (120x97x104: 26 us against 26 + about 5 in three launches).
 template <class F>
-__global__ void __launch_bounds__(256, 3) k3p_dir_apply(Dom3 d, const double *__restrict__ CX, const double *__restrict__ CY,
-                                                        const double *__restrict__ CZ, const double *__restrict__ Z,
-                                                        double *D0, double *D1, double *__restrict__ PHI,
-                                                        double *__restrict__ AD, const int *gate, double *part, Sc3 *sc, F then)
+__global__ void __launch_bounds__(256, 4) k3p_apply(Dom3 d, const double *__restrict__ CX, const double *__restrict__ CY,
+                                                    const double *__restrict__ CZ, const double *__restrict__ X,
+                                                    double *__restrict__ AD, const int *gate, double *part, Sc3 *sc,
+                                                    F then)
 {
-    __shared__ double2 tile[2][8][32];
     if (gate && *gate == 0) return;
     const int ni = d.NX - 1, nj = d.NY - 1, nk = d.NZ - 1;
-    const int tx = threadIdx.x, ty = threadIdx.y, i = 2 * (blockIdx.x * 32 + tx), j = blockIdx.y * 8 + ty;
-    const int done = sc->p_iter;
-    const bool first = done == 0, live = i < ni && j < nj, two = i + 1 < ni;
-    const double *__restrict__ DO = (done & 1) ? D1 : D0;
-    double *__restrict__ DN = (done & 1) ? D0 : D1;
-    const double beta = sc->p_beta, alpha = first ? 0.0 : sc->p_alpha;
+    const int i = 2 * (blockIdx.x * 32 + threadIdx.x), j = blockIdx.y * 8 + threadIdx.y;
     double acc[1] = {0.0};
-    // the neighbours' sources under the pressure ghost rules (copies), from the
-    // maps once per thread
-    const Map3 &m = d.map[K_PRESSURE];
-    const int il = live ? i : 0, jl = live ? j : 0;
-    const int row = jl * d.P, oc = row + il, ow = row + m.x.src[il - 1 + NG], oe = row + m.x.src[il + (two ? 2 : 1) + NG];
-    const int os = m.y.src[jl - 1 + NG] * d.P + il, on = m.y.src[jl + 1 + NG] * d.P + il;
-    const bool we = tx == 0, ee = tx == 31 || i + 2 >= ni, se = ty == 0, ne = ty == 7 || j + 1 >= nj;   // the tile's edges
-    auto one = [&](const double *z, const double *o, int q) { return first ? z[q] : z[q] + beta * o[q]; };
-    auto form = [&](double2 z, double2 o) { return first ? z : make_double2(z.x + beta * o.x, z.y + beta * o.y); };
-    const double2 zero = make_double2(0.0, 0.0);
-    auto old = [&](const double *p) { return first ? zero : ld2(p); };
-    const int k0 = blockIdx.z * PKD, k1 = k0 + PKD < nk ? k0 + PKD : nk;
-    double2 bk = zero, c = zero, o = zero, czm = zero;
-    if (live) {
-        const long long pb = m.z.src[k0 - 1 + NG] * d.S + oc, q = k0 * d.S + oc;
-        o = old(DO + q);
-        bk = form(ld2(Z + pb), old(DO + pb));
-        c = form(ld2(Z + q), o);
-        czm = ld2(CZ + q - d.S);
-    }
+    if (i < ni && j < nj) {
+        const bool two = i + 1 < ni;
 #pragma unroll 1
-    for (int k = k0; k < k1; k++) {
-        const long long pl = k * d.S, q = pl + oc, pf = m.z.src[k + 1 + NG] * d.S + oc;
-        double2 f = zero, fo = zero, cx = zero, cy = zero, cz = zero, cym = zero, ph = zero, s = zero, n = zero;
-        double w = 0.0, e = 0.0, cxm = 0.0;
-        if (live) {
-            f = ld2(Z + pf);
-            fo = old(DO + pf);
-            cx = ld2(CX + q);
-            cy = ld2(CY + q);
-            cz = ld2(CZ + q);
-            cym = ld2(CY + q - d.P);
-            cxm = CX[q - 1];
-            if (!first) ph = ld2(PHI + q);
-            if (we) w = one(Z + pl, DO + pl, ow);
-            if (ee) e = one(Z + pl, DO + pl, oe);
-            if (se) s = form(ld2(Z + pl + os), old(DO + pl + os));
-            if (ne) n = form(ld2(Z + pl + on), old(DO + pl + on));
-        }
-        tile[k & 1][ty][tx] = c;
-        const double wl = __shfl_up_sync(0xffffffffu, c.y, 1), el = __shfl_down_sync(0xffffffffu, c.x, 1);
-        __syncthreads();
-        if (live) {
-            if (!we) w = wl;
-            if (!ee) e = el;
-            if (!se) s = tile[k & 1][ty - 1][tx];
-            if (!ne) n = tile[k & 1][ty + 1][tx];
-            const double2 fn = form(f, fo);
-            const double e0 = two ? c.y : e;
-            const double v0 = cx.x * (e0 - c.x) - cxm * (c.x - w) + cy.x * (n.x - c.x) - cym.x * (c.x - s.x) +
-                              cz.x * (fn.x - c.x) - czm.x * (c.x - bk.x);
-            const double ad0 = 1.0 * v0;
+        for (int kk = 0; kk < PKB; kk++) {
+            const int k = blockIdx.z * PKB + kk;
+            if (k >= nk) break;
+            const long long q = at(d, i, j, k);
+            // a row's single last cell goes with the pairs, its second cell (the half
+            // cell beyond the row) neither summed nor stored (on a path of its own the
+            // rest of the warp waited for it: 127^3 79.7 -> 67.6 us an iteration)
+            const double2 c = ld2(X + q);
+            const double w0 = (i >= 1) ? X[q - 1] : rd<K_PRESSURE>(d, X, i - 1, j, k);
+            const int ie = two ? i + 2 : i + 1;
+            const double e1 = (ie <= ni - 1) ? X[q + 2] : rd<K_PRESSURE>(d, X, ie, j, k), e0 = two ? c.y : e1;
+            double s0, s1, n0, n1, b0, b1, f0, f1;
+            p_pair(d, X, i, j - 1, k, s0, s1);
+            p_pair(d, X, i, j + 1, k, n0, n1);
+            p_pair(d, X, i, j, k - 1, b0, b1);
+            p_pair(d, X, i, j, k + 1, f0, f1);
+            const double2 cx = ld2(CX + q), cy = ld2(CY + q), cz = ld2(CZ + q);
+            const double2 cym = ld2(CY + q - d.P), czm = ld2(CZ + q - d.S);
+            const double cxm = CX[q - 1];
+            const double v0 = cx.x * (e0 - c.x) - cxm * (c.x - w0) + cy.x * (n0 - c.x) - cym.x * (c.x - s0) +
+                              cz.x * (f0 - c.x) - czm.x * (c.x - b0);
+            const double v1 = cx.y * (e1 - c.y) - cx.x * (c.y - c.x) + cy.y * (n1 - c.y) - cym.y * (c.y - s1) +
+                              cz.y * (f1 - c.y) - czm.y * (c.y - b1);
+            const double ad0 = 1.0 * v0, ad1 = 1.0 * v1;
             acc[0] += c.x * ad0;
             if (two) {
-                const double v1 = cx.y * (e - c.y) - cx.x * (c.y - c.x) + cy.y * (n.y - c.y) - cym.y * (c.y - s.y) +
-                                  cz.y * (fn.y - c.y) - czm.y * (c.y - bk.y);
-                const double ad1 = 1.0 * v1;
-                acc[0] += c.y * ad1;
-                if (!first) st2(PHI + q, ph.x + alpha * o.x, ph.y + alpha * o.y);
-                st2(DN + q, c.x, c.y);
                 st2(AD + q, ad0, ad1);
-            } else {   // a row's single last cell
-                if (!first) PHI[q] = ph.x + alpha * o.x;
-                DN[q] = c.x;
+                acc[0] += c.y * ad1;
+            } else {
                 AD[q] = ad0;
             }
-            bk = c;
-            c = fn;
-            o = fo;
-            czm = cz;
         }
     }
     block_sum_then(acc, part, sc, then);
 }
 
-// Second pass: r -= alpha Ad, r.Mr, and z = M r where that is the
-// preconditioner (ZW).
-template <bool ZW, class F>
-__global__ void __launch_bounds__(256) k3p_resid(Dom3 d, double *__restrict__ R, const double *__restrict__ AD,
-                                                 const double *__restrict__ M, double *__restrict__ Z, const int *gate, Sc3 *sc,
-                                                 double *part, F then)
+template <class F>
+__global__ void __launch_bounds__(256) k3p_update(Dom3 d, double *__restrict__ PHI, double *__restrict__ R,
+                                                  const double *__restrict__ DD, const double *__restrict__ AD,
+                                                  const double *__restrict__ M, const int *gate, Sc3 *sc,
+                                                  double *part, F then)
 {
     if (gate && *gate == 0) return;
     const int ni = d.NX - 1, nj = d.NY - 1, nk = d.NZ - 1;
@@ -307,21 +279,44 @@ __global__ void __launch_bounds__(256) k3p_resid(Dom3 d, double *__restrict__ R,
             if (k >= nk) break;
             const long long q = at(d, i, j, k);
             if (!two) {
-                const double r = R[q] - alpha * AD[q], z = r * M[q];
+                PHI[q] += alpha * DD[q];
+                const double r = R[q] - alpha * AD[q];
                 R[q] = r;
-                if (ZW) Z[q] = z;
-                acc[0] += r * z;
+                acc[0] += r * (r * M[q]);
                 continue;
             }
-            const double2 r = ld2(R + q), ad = ld2(AD + q), m = ld2(M + q);
-            const double r0 = r.x - alpha * ad.x, r1 = r.y - alpha * ad.y, z0 = r0 * m.x, z1 = r1 * m.y;
+            const double2 x = ld2(PHI + q), dd = ld2(DD + q), r = ld2(R + q), ad = ld2(AD + q), m = ld2(M + q);
+            st2(PHI + q, x.x + alpha * dd.x, x.y + alpha * dd.y);
+            const double r0 = r.x - alpha * ad.x, r1 = r.y - alpha * ad.y;
             st2(R + q, r0, r1);
-            if (ZW) st2(Z + q, z0, z1);
-            acc[0] += r0 * z0;
-            acc[0] += r1 * z1;
+            acc[0] += r0 * (r0 * m.x);
+            acc[0] += r1 * (r1 * m.y);
         }
     }
     block_sum_then(acc, part, sc, then);
+}
+
+__global__ void __launch_bounds__(256) k3p_dir(Dom3 d, const double *__restrict__ R, const double *__restrict__ M,
+                                               double *__restrict__ DD, const int *gate, const Sc3 *sc)
+{
+    if (gate && *gate == 0) return;
+    const int ni = d.NX - 1, nj = d.NY - 1, nk = d.NZ - 1;
+    const int i = 2 * (blockIdx.x * 32 + threadIdx.x), j = blockIdx.y * 8 + threadIdx.y;
+    if (i >= ni || j >= nj) return;
+    const double beta = sc->p_beta;
+    const bool two = i + 1 < ni;
+#pragma unroll
+    for (int kk = 0; kk < PKB; kk++) {
+        const int k = blockIdx.z * PKB + kk;
+        if (k >= nk) break;
+        const long long q = at(d, i, j, k);
+        if (!two) {
+            DD[q] = R[q] * M[q] + beta * DD[q];
+            continue;
+        }
+        const double2 r = ld2(R + q), m = ld2(M + q), dd = ld2(DD + q);
+        st2(DD + q, r.x * m.x + beta * dd.x, r.y * m.y + beta * dd.y);
+    }
 }
 
 // The momentum PCG's two passes over the faces of component C (one face per
@@ -344,8 +339,10 @@ __global__ void __launch_bounds__(256, 4) k3v_dir_op(Dom3 d, Range r, double iRe
     double *__restrict__ DN = (done & 1) ? D0 : D1;
     const double beta = sc->v_beta, alpha = first ? 0.0 : sc->v_alpha;
     double acc[1] = {0.0};
-    // neighbours as in k3p_dir_apply; the sources and multipliers (y walls) under
-    // the ghost rule KC once per thread
+    // east and west neighbours come from the neighbouring lanes, north and south from
+    // the tile in shared memory, and only the tile's edges form a neighbour's
+    // direction themselves; the sources and multipliers (y walls) under the ghost
+    // rule KC once per thread
     const int tx = threadIdx.x, ty = threadIdx.y;
     const bool live = i < r.i1 && j < r.j1;
     const Map3 &m = d.map[KC];
@@ -756,6 +753,29 @@ __global__ void __launch_bounds__(XT, 2) k3s_inv_x(Dom3 d, SpecDims sd, const do
     block_sum_then(acc, part, sc, then);
 }
 
+// d = z + beta d (the spectral form's direction)
+__global__ void __launch_bounds__(256) k3p_dir_z(Dom3 d, const double *__restrict__ Z, double *__restrict__ DD,
+                                                 const int *gate, const Sc3 *sc)
+{
+    if (gate && *gate == 0) return;
+    const int ni = d.NX - 1, nj = d.NY - 1, nk = d.NZ - 1;
+    const int i = 2 * (blockIdx.x * 32 + threadIdx.x), j = blockIdx.y * 8 + threadIdx.y;
+    if (i >= ni || j >= nj) return;
+    const double beta = sc->p_beta;
+    const bool two = i + 1 < ni;
+    for (int kk = 0; kk < PKB; kk++) {
+        const int k = blockIdx.z * PKB + kk;
+        if (k >= nk) break;
+        const long long q = at(d, i, j, k);
+        if (!two) {
+            DD[q] = Z[q] + beta * DD[q];
+            continue;
+        }
+        const double2 z = ld2(Z + q), dd = ld2(DD + q);
+        st2(DD + q, z.x + beta * dd.x, z.y + beta * dd.y);
+    }
+}
+
 // host block (reference layout) <-> padded field
 __global__ void k3_unpack(Dom3 d, double *fld, const double *blk, int ng)
 {
@@ -866,10 +886,10 @@ struct GpuExec {
         note();
         pend.mask = 0;
     }
-    // the pressure PCG iteration's two passes (k3p_*)
-    static dim3 pgrid(const Dom3 &d, int planes)
+    // the pressure PCG iteration's three passes (k3p_*)
+    static dim3 pgrid(const Dom3 &d)
     {
-        return dim3((unsigned)((d.NX - 1 + 63) / 64), (unsigned)((d.NY - 1 + 7) / 8), (unsigned)((d.NZ - 1 + planes - 1) / planes));
+        return dim3((unsigned)((d.NX - 1 + 63) / 64), (unsigned)((d.NY - 1 + 7) / 8), (unsigned)((d.NZ - 1 + PKB - 1) / PKB));
     }
     // the momentum PCG's (k3v_*)
     static dim3 vgrid(const Range &r)
@@ -880,16 +900,27 @@ struct GpuExec {
     // reductions of the solves do not touch
     double *last_slot() { return part + (size_t)(NSLOT - 1) * pstride; }
     template <class F>
-    void p_dir_apply(const Dom3 &d, const double *CX, const double *CY, const double *CZ, const double *Z, double *D0, double *D1,
-                     double *PHI, double *AD, const int *gate, F then)
+    void p_apply(const Dom3 &d, const double *CX, const double *CY, const double *CZ, const double *X, double *AD,
+                 const int *gate, F then)
     {
-        k3p_dir_apply<<<pgrid(d, PKD), dim3(32, 8), 0, stream>>>(d, CX, CY, CZ, Z, D0, D1, PHI, AD, gate, last_slot(), sc, then);
+        k3p_apply<<<pgrid(d), dim3(32, 8), 0, stream>>>(d, CX, CY, CZ, X, AD, gate, last_slot(), sc, then);
         note();
     }
-    template <bool ZW, class F>
-    void p_resid(const Dom3 &d, double *R, const double *AD, const double *M, double *Z, const int *gate, F then)
+    template <class F>
+    void p_update(const Dom3 &d, double *PHI, double *R, const double *DD, const double *AD, const double *M,
+                  const int *gate, F then)
     {
-        k3p_resid<ZW><<<pgrid(d, PKB), dim3(32, 8), 0, stream>>>(d, R, AD, M, Z, gate, sc, last_slot(), then);
+        k3p_update<<<pgrid(d), dim3(32, 8), 0, stream>>>(d, PHI, R, DD, AD, M, gate, sc, last_slot(), then);
+        note();
+    }
+    void p_dir(const Dom3 &d, const double *R, const double *M, double *DD, const int *gate)
+    {
+        k3p_dir<<<pgrid(d), dim3(32, 8), 0, stream>>>(d, R, M, DD, gate, sc);
+        note();
+    }
+    void p_dir_z(const Dom3 &d, const double *Z, double *DD, const int *gate)
+    {
+        k3p_dir_z<<<pgrid(d), dim3(32, 8), 0, stream>>>(d, Z, DD, gate, sc);
         note();
     }
     template <int C, int KC, class F>

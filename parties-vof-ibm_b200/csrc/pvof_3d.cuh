@@ -393,7 +393,7 @@ enum F3 {
     F3_VR, F3_VD, F3_VAD, F3_VDIAG,
     F3_FSO_X, F3_FSO_Y, F3_FSO_Z, F3_FSN_X, F3_FSN_Y, F3_FSN_Z,
     F3_PCX, F3_PCY, F3_PCZ, F3_PZ, F3_PSM,
-    F3_VFT, F3_VMU, F3_VMA, F3_VMB, F3_VZ, F3_VD2, F3_VZ_V, F3_VD2_V, F3_PD2,
+    F3_VFT, F3_VMU, F3_VMA, F3_VMB, F3_VZ, F3_VD2, F3_VZ_V, F3_VD2_V,
     F3_COUNT
 };
 
@@ -1198,7 +1198,7 @@ struct Box3 {
         const Dom3 d = this->d;
         Sc3 *sc = x.sc;
         const double *B = f[F3_PRHS], *M = f[F3_PM], *CX = f[F3_PCX], *CY = f[F3_PCY], *CZ = f[F3_PCZ];
-        double *PHI = f[F3_DP], *R = f[F3_PR], *D0 = f[F3_PD], *D1 = f[F3_PD2], *AD = f[F3_PAD], *Z = f[F3_PZ], *SM = f[F3_PSM];
+        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD], *Z = f[F3_PZ], *SM = f[F3_PSM];
         const double tol = p.P_CG_ETOL;
         const int maxit = p.P_CG_MAXIT;
         const Range cr = cells_range(d);
@@ -1209,11 +1209,12 @@ struct Box3 {
             SM[q] = sqrt(M[q]);
             return Vec<1>{{r * (r * M[q])}};
         });
-        // z = P r and gamma = r.z
+        // z = P r and gamma = r.z, then d = z
         x.spec_apply(d, R, SM, Z, nullptr, [=] __host__ __device__(Sc3 * s, double rz) {
             s->p_gamma = rz;
             s->p_beta = 0.0;
         });
+        x.p_dir_z(d, Z, DD, nullptr);
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->p_gamma_new = s->sum[0][0];   // r.Mr: the stopping quantity
             s->p_iter = 0;
@@ -1226,29 +1227,28 @@ struct Box3 {
         const int *gate = &sc->p_active;
         for (int it = 0, chunk = CHUNK; it < maxit; it += chunk, chunk = next_chunk(chunk)) {
             for (int q = 0; q < chunk && it + q < maxit; q++) {
-                x.p_dir_apply(d, CX, CY, CZ, Z, D0, D1, PHI, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
+                x.p_apply(d, CX, CY, CZ, DD, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
                     s->p_alpha = s->p_gamma / (dAd + 1e-300);
                 });
-                x.template p_resid<false>(d, R, AD, M, Z, gate, [=] __host__ __device__(Sc3 * s, double rMr) {
+                x.p_update(d, PHI, R, DD, AD, M, gate, [=] __host__ __device__(Sc3 * s, double rMr) {
                     s->p_iter++;
                     s->p_gamma_new = rMr;
                     if (sqrt(rMr) < s->p_tol) s->p_active = 0;
                 });
-                // z = P r, r.z and the direction's coefficient
+                // z = P r, r.z and the direction's coefficient, then d = z + beta d
                 x.spec_apply(d, R, SM, Z, gate, [=] __host__ __device__(Sc3 * s, double g) {
                     s->p_beta = g / (s->p_gamma + 1e-300);
                     s->p_gamma = g;
                     if (s->p_iter >= s->p_maxit) s->p_active = 0;
                 });
+                x.p_dir_z(d, Z, DD, gate);
             }
             if (!x.read_int(gate)) break;
         }
         const int *ran = &sc->p_ran;
         const double count = (double)((long long)(d.NX - 1) * (d.NY - 1) * (d.NZ - 1));
         x.template reduce<1>(cr, ran, 0, [=] __host__ __device__(int i, int j, int k) {
-            const long long q = at(d, i, j, k);
-            if (sc->p_iter > 0) PHI[q] += sc->p_alpha * ((sc->p_iter & 1) ? D1 : D0)[q];   // the last iteration's update
-            return Vec<1>{{PHI[q]}};
+            return Vec<1>{{PHI[at(d, i, j, k)]}};
         });
         x.scalar(ran, [=] __host__ __device__(Sc3 * s) { s->p_avg = s->sum[0][0] / count; });
         x.cells(cr, ran, [=] __host__ __device__(int i, int j, int k) { PHI[at(d, i, j, k)] -= sc->p_avg; });
@@ -1268,7 +1268,7 @@ struct Box3 {
         const Dom3 d = this->d;
         Sc3 *sc = x.sc;
         const double *B = f[F3_PRHS], *M = f[F3_PM], *CX = f[F3_PCX], *CY = f[F3_PCY], *CZ = f[F3_PCZ];
-        double *PHI = f[F3_DP], *R = f[F3_PR], *D0 = f[F3_PD], *D1 = f[F3_PD2], *AD = f[F3_PAD], *Z = f[F3_PZ];
+        double *PHI = f[F3_DP], *R = f[F3_PR], *DD = f[F3_PD], *AD = f[F3_PAD];
         const double tol = p.P_CG_ETOL;
         const int maxit = p.P_CG_MAXIT;
         const Range cr = cells_range(d);
@@ -1277,13 +1277,12 @@ struct Box3 {
             const double r = B[q] - p_apply_st(d, CX, CY, CZ, PHI, i, j, k);
             R[q] = r;
             const double z = r * M[q];
-            Z[q] = z;
+            DD[q] = z;
             return Vec<1>{{r * z}};
         });
         x.scalar(nullptr, [=] __host__ __device__(Sc3 * s) {
             s->p_gamma = s->sum[0][0];
             s->p_gamma_new = s->p_gamma;
-            s->p_beta = 0.0;
             s->p_iter = 0;
             s->p_maxit = maxit;
             s->p_tol = tol;
@@ -1294,14 +1293,14 @@ struct Box3 {
         const int *gate = &sc->p_active;
         for (int it = 0, chunk = CHUNK; it < maxit; it += chunk, chunk = next_chunk(chunk)) {
             for (int q = 0; q < chunk && it + q < maxit; q++) {
-                // phi += alpha d of the iteration before, d = z + beta d, AD = A d and
-                // d.AD, then the step length from the finished sum
-                x.p_dir_apply(d, CX, CY, CZ, Z, D0, D1, PHI, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
+                // AD = A d and d.AD (the executor's streaming form of p_apply_st),
+                // then the step length from the finished sum
+                x.p_apply(d, CX, CY, CZ, DD, AD, gate, [=] __host__ __device__(Sc3 * s, double dAd) {
                     s->p_alpha = s->p_gamma / (dAd + 1e-30);
                 });
-                // r -= alpha AD, z = M r and r.z, then the stopping test and the
-                // direction's coefficient
-                x.template p_resid<true>(d, R, AD, M, Z, gate, [=] __host__ __device__(Sc3 * s, double rz) {
+                // phi += alpha d, r -= alpha AD and r.(M r), then the stopping test
+                // and the direction's coefficient
+                x.p_update(d, PHI, R, DD, AD, M, gate, [=] __host__ __device__(Sc3 * s, double rz) {
                     s->p_iter++;
                     s->p_gamma_new = rz;
                     if (sqrt(s->p_gamma_new) < s->p_tol) {
@@ -1312,6 +1311,8 @@ struct Box3 {
                         if (s->p_iter >= s->p_maxit) s->p_active = 0;
                     }
                 });
+                // d = M r + beta d
+                x.p_dir(d, R, M, DD, gate);
             }
             if (!x.read_int(gate)) break;
         }
@@ -1319,9 +1320,7 @@ struct Box3 {
         const int *ran = &sc->p_ran;
         const double count = (double)((long long)(d.NX - 1) * (d.NY - 1) * (d.NZ - 1));
         x.template reduce<1>(cr, ran, 0, [=] __host__ __device__(int i, int j, int k) {
-            const long long q = at(d, i, j, k);
-            if (sc->p_iter > 0) PHI[q] += sc->p_alpha * ((sc->p_iter & 1) ? D1 : D0)[q];   // the last iteration's update
-            return Vec<1>{{PHI[q]}};
+            return Vec<1>{{PHI[at(d, i, j, k)]}};
         });
         x.scalar(ran, [=] __host__ __device__(Sc3 * s) { s->p_avg = s->sum[0][0] / count; });
         x.cells(cr, ran, [=] __host__ __device__(int i, int j, int k) { PHI[at(d, i, j, k)] -= sc->p_avg; });
