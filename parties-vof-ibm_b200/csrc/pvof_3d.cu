@@ -348,7 +348,9 @@ __global__ void __launch_bounds__(256, 4) k3v_dir_op(Dom3 d, Range r, double iRe
     const Map3 &m = d.map[KC];
     const int il = live ? i : r.i0, jl = live ? j : r.j0;
     const int row = jl * d.P, oc = row + il, ow = row + m.x.src[il - 1 + NG], oe = row + m.x.src[il + 1 + NG];
-    const int os = m.y.src[jl - 1 + NG] * d.P + il, on = m.y.src[jl + 1 + NG] * d.P + il;
+    // the walls' faces of v keep their place under the rule and are no unknowns: zero
+    const int js = m.y.src[jl - 1 + NG], jn = m.y.src[jl + 1 + NG], os = js * d.P + il, on = jn * d.P + il;
+    const bool hs = js >= r.j0 && js < r.j1, hn = jn >= r.j0 && jn < r.j1;
     const double ms = m.y.mul[jl - 1 + NG], mn = m.y.mul[jl + 1 + NG];
     const bool we = tx == 0, ee = tx == 31 || i + 1 >= r.i1, se = ty == 0, ne = ty == 7 || j + 1 >= r.j1;
     auto dir = [&](long long q) { return first ? Z[q] : Z[q] + beta * DO[q]; };
@@ -366,8 +368,8 @@ __global__ void __launch_bounds__(256, 4) k3v_dir_op(Dom3 d, Range r, double iRe
             f = dir(m.z.src[k + 1 + NG] * d.S + oc);
             if (we) w = dir(pl + ow);
             if (ee) e = dir(pl + oe);
-            if (se) s = ms * dir(pl + os);
-            if (ne) n = mn * dir(pl + on);
+            if (se && hs) s = ms * dir(pl + os);
+            if (ne && hn) n = mn * dir(pl + on);
             if (!first) xo = X[q] + alpha * DO[q];
         }
         tile[k & 1][ty][tx] = c;
@@ -1173,15 +1175,12 @@ int create(const pvof_grid_desc *g, const pvof_params *p, int device, Handle **o
     auto bail = [&](int rc) { destroy(h); return rc; };
     if (cudaStreamCreateWithFlags(&x.stream, cudaStreamNonBlocking) != cudaSuccess) return bail(fail(PVOF_ECUDA, "stream"));
     // fields (zeroed once: never-written positions read as the reference's zero-initialised arrays)
-    const int nfields = F3_COUNT + 2;
+    const int nfields = F3_COUNT;
     if (cudaMalloc(&h->mem, x.field_elems * sizeof(double) * nfields) != cudaSuccess)
         return bail(fail(PVOF_ENOMEM, "device memory for the 3D fields"));
     if (cudaMemsetAsync(h->mem, 0, x.field_elems * sizeof(double) * nfields, x.stream) != cudaSuccess)
         return bail(fail(PVOF_ECUDA, "memset"));
     for (int q = 0; q < F3_COUNT; q++) b.f[q] = h->mem + (size_t)q * x.field_elems + x.origin;
-    b.vd[0] = b.f[F3_VD];
-    b.vd[1] = h->mem + (size_t)F3_COUNT * x.field_elems + x.origin;
-    b.vd[2] = h->mem + (size_t)(F3_COUNT + 1) * x.field_elems + x.origin;
     // tables: metrics per axis (8 arrays), weights, map multipliers; map sources
     HostAxis ax[3];
     const bool per[3] = {true, false, true};

@@ -393,8 +393,11 @@ enum F3 {
     F3_VR, F3_VD, F3_VAD, F3_VDIAG,
     F3_FSO_X, F3_FSO_Y, F3_FSO_Z, F3_FSN_X, F3_FSN_Y, F3_FSN_Z,
     F3_PCX, F3_PCY, F3_PCZ, F3_PZ, F3_PSM,
-    F3_VFT, F3_VMU, F3_VMA, F3_VMB, F3_VZ, F3_VD2, F3_VZ_V, F3_VD2_V,
-    F3_COUNT
+    F3_COUNT,
+    // fields of the momentum solve in storage that only the pressure solve and the
+    // biharmonic solve use, each from its own start to its end within a substep;
+    // none of them reads a position of these that it has not written
+    F3_VFT = F3_PR, F3_VMU = F3_PD, F3_VMA = F3_PAD, F3_VMB = F3_PZ, F3_VD2 = F3_PSM, F3_VZ = F3_AP
 };
 
 // the owned index boxes of the reference's loops (e.g. Velocity.c:395-410,
@@ -776,7 +779,6 @@ struct Box3 {
     pvof_grid_desc g;
     pvof_params p;
     double *f[F3_COUNT] = {};
-    double *vd[3] = {};       // velocity CG directions, one per component
     int stage = 0;
     double dt = 0.0, time = 0.0, clamp_total = 0.0;
     bool initialized = false;
@@ -1092,9 +1094,7 @@ struct Box3 {
         const double *CL = f[F3_CL], *RHS = f[F3_U_RHS + 3 * C];
         double *DATA = f[F3_U + C], *R = f[F3_VR], *AD = f[F3_VAD], *DG = f[F3_VDIAG];
         double *FT = f[F3_VFT], *MU = f[F3_VMU], *MA = f[F3_VMA], *MB = f[F3_VMB];
-        // the direction's wall faces of v read as stored (zero): fields that no
-        // other component writes
-        double *D0 = vd[C], *D1 = f[C == 1 ? F3_VD2_V : F3_VD2], *Z = f[C == 1 ? F3_VZ_V : F3_VZ];
+        double *D0 = f[F3_VD], *D1 = f[F3_VD2], *Z = f[F3_VZ];
         const double iRe = 1.0 / p.Re, alpha_k = bet(stage), dt = this->dt;
         const double EPS = p.velocity_cg_unregularized ? 0.0 : 1e-14;
         const int NX = d.NX, NY = d.NY, NZ = d.NZ;
