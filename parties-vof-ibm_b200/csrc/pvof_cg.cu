@@ -559,7 +559,11 @@ __device__ __forceinline__ void cg_pressure_resident(const PresArgs &A, const Ra
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = iters; A.scal->p_res = sqrt(gamma_new); }
 }
 
-template <bool PAIR>
+// WEIGHTS: the face weights come from the planes A.bx / A.by, filled by the
+// set-up phase; otherwise each is computed where it is needed (the no-allocation
+// entry point on a device too small for a cell per thread: its scratch has no
+// room for them).
+template <bool PAIR, bool WEIGHTS>
 __device__ __forceinline__ void cg_pressure(const PresArgs &A)
 {
     const Dom &d = A.d;
@@ -573,7 +577,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     const double *__restrict__ bx = A.bx;
     const double *__restrict__ by = A.by;
     Slots sl{reinterpret_cast<unsigned long long *>(A.partials), &A.scal->error, gridDim.x, blockIdx.x, 1, 0};
-    if (!PAIR && R.n <= nth) {   // one cell per thread
+    if (!PAIR && WEIGHTS && R.n <= nth) {   // one cell per thread
         cg_pressure_resident(A, R);
         return;
     }
@@ -582,7 +586,7 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     for (int q = tid; q < R.n; q += nth) {
         int i, j;
         R.ij(q, i, j);
-        pressure_face_weights(d, rho, A.bx, A.by, i, j);
+        if (WEIGHTS) pressure_face_weights(d, rho, A.bx, A.by, i, j);
         double ad = pressure_op(d, rho, i, j, [&](int a, int b) { return remap(A.mp, A.phi, P, NX, NY, a, b); });
         // the axisymmetric right-hand side carries the row weight r_c of the
         // operator (psolve_hypre.c:184-200)
@@ -622,7 +626,14 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
             vn = zp[cN] + bt * dold[cN];
             vs = zp[cS] + bt * dold[cS];
         }
-        const double bxm = bx[cC - 1], bxp = bx[cC], bym = by[cC - P], byp = by[cC];
+        double bxm, bxp, bym, byp;
+        if (WEIGHTS) {
+            bxm = bx[cC - 1]; bxp = bx[cC]; bym = by[cC - P]; byp = by[cC];
+        } else {
+            const double r0 = rho[cC];
+            bxm = 2.0 / (r0 + rho[cC - 1]); bxp = 2.0 / (r0 + rho[cC + 1]);
+            bym = 2.0 / (r0 + rho[cC - P]); byp = 2.0 / (r0 + rho[cC + P]);
+        }
         double cxm, cxp, cym, cyp;
         face_coeffs(d, i, bxm, bxp, bym, byp, cxm, cxp, cym, cyp);
         const double val = cxp * (ve - vc) - cxm * (vc - vw) + cyp * (vn - vc) - cym * (vc - vs);
@@ -791,12 +802,14 @@ __device__ __forceinline__ void cg_pressure(const PresArgs &A)
     if (blockIdx.x == 0 && threadIdx.x == 0) { A.scal->p_iters = iters; A.scal->p_res = sqrt(gamma_new); }
 }
 
-// the no-allocation entry point's solve: at most one cell per resident thread
+// the no-allocation entry point's solve: at most one cell per resident thread, or
+// a walk of the range where the device holds fewer threads
 __global__ void __launch_bounds__(512) k_cg_pressure(PresArgs A)
 {
     cg_pressure_resident(A, Range{0, 0, A.d.NX - 1, (A.d.NX - 1) * (A.d.NY - 1)});
 }
-__global__ void __launch_bounds__(512, 2) k_cg_pressure_fw(PresArgs A) { cg_pressure<false>(A); }
-__global__ void __launch_bounds__(512, 2) k_cg_pressure_fwp(PresArgs A) { cg_pressure<true>(A); }
+__global__ void __launch_bounds__(512) k_cg_pressure_walk(PresArgs A) { cg_pressure<false, false>(A); }
+__global__ void __launch_bounds__(512, 2) k_cg_pressure_fw(PresArgs A) { cg_pressure<false, true>(A); }
+__global__ void __launch_bounds__(512, 2) k_cg_pressure_fwp(PresArgs A) { cg_pressure<true, true>(A); }
 
 }  // namespace pvof

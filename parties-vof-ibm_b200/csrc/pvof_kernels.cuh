@@ -285,6 +285,7 @@ __global__ void k_cg_biharmonic_fly(BihArgs A);
 __global__ void k_cg_velocity(VelArgs A);
 __global__ void k_cg_velocity_res(VelArgs A);
 __global__ void k_cg_pressure(PresArgs A);
+__global__ void k_cg_pressure_walk(PresArgs A);
 __global__ void k_cg_pressure_fw(PresArgs A);
 __global__ void k_cg_pressure_fwp(PresArgs A);
 

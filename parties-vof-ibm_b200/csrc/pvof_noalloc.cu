@@ -19,6 +19,7 @@
 //   * the first call on a device looks up the array's device address
 //     (cudaGetSymbolAddress) with that device current; make that first call
 //     before any stream capture.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -34,7 +35,7 @@ constexpr int NOALLOC_MAX_BLOCKS = (int)((NOALLOC_PLANE_MAX + NOALLOC_THREADS - 
 constexpr size_t NOALLOC_AXIS_LEN = NOALLOC_AXIS_MAX + 1 + 2 * NG;  // entries of a per-axis table
 
 // layout of the scratch array, in doubles
-constexpr size_t NA_PLANES = 6;  // M, res, dir, dir2, z, Ad
+constexpr size_t NA_PLANES = 6;  // M, z; res, dir, dir2, Ad where a thread has several cells
 constexpr size_t NA_OFF_PART = NA_PLANES * NOALLOC_PLANE_MAX;
 constexpr size_t NA_OFF_SCAL = NA_OFF_PART + SLOT_DOUBLES * (size_t)(NOALLOC_MAX_BLOCKS + 1);
 constexpr size_t NA_SCAL_LEN = (sizeof(DevScalars) + sizeof(double) - 1) / sizeof(double);
@@ -51,7 +52,7 @@ namespace {
 
 struct DeviceScratch {
     double *base = nullptr;
-    int coop_blocks = 0;
+    int resident_blocks = 0, walk_blocks = 0;   // co-resident blocks of the two forms of the solve
 };
 
 std::mutex g_mu;
@@ -60,7 +61,7 @@ DeviceScratch g_dev[64];
 int na_err(int code, const char *msg);
 
 // per-device set-up: device address of the scratch array and the
-// co-resident block count of the grid-wide pressure solver
+// co-resident block counts of the pressure solver's two forms
 int scratch_for_device(int dev, DeviceScratch &out)
 {
     std::lock_guard<std::mutex> lock(g_mu);
@@ -70,12 +71,14 @@ int scratch_for_device(int dev, DeviceScratch &out)
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || p == nullptr) return na_err(PVOF_ECUDA, "cudaGetSymbolAddress of the scratch array failed");
-        int nsm = 0, occ = 0;
+        int nsm = 0, occ = 0, occ_walk = 0;
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_pressure, NOALLOC_THREADS, 0) != cudaSuccess || occ < 1)
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_pressure, NOALLOC_THREADS, 0) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_walk, k_cg_pressure_walk, NOALLOC_THREADS, 0) != cudaSuccess ||
+            occ < 1 || occ_walk < 1)
             return na_err(PVOF_ECUDA, "occupancy query failed");
-        int nb = occ * nsm;
-        s.coop_blocks = nb < NOALLOC_MAX_BLOCKS ? nb : NOALLOC_MAX_BLOCKS;
+        s.resident_blocks = std::min(occ * nsm, NOALLOC_MAX_BLOCKS);
+        s.walk_blocks = std::min(occ_walk * nsm, NOALLOC_MAX_BLOCKS);
         s.base = (double *)p;
     }
     out = s;
@@ -144,10 +147,11 @@ using namespace pvof;
 
 extern "C" const char *pvof_noalloc_last_error(void) { return g_na_msg; }
 
-// See the file comment and include/pvof.h.
-extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const pvof_params *params,
-                                              const double *rho, const double *rhs, double *phi, void *stream,
-                                              int *iterations, double *residual)
+// The solve on at most `most` blocks.  The entry point below gives no limit of
+// its own; tests give one, to run the form for devices that hold fewer threads
+// than a grid has cells.
+extern "C" int pvof_noalloc_solve(const pvof_grid_desc *grid, const pvof_params *params, const double *rho, const double *rhs,
+                                  double *phi, void *stream, int *iterations, double *residual, int most)
 {
     if (!grid || !params || !rho || !rhs || !phi) return na_err(PVOF_EINVAL, "null argument");
     if (grid->ghost_nodes != NG || grid->NZM != 1 ||
@@ -198,8 +202,8 @@ extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const 
     mw.x = {src + 2 * NOALLOC_AXIS_LEN, mul + 2 * NOALLOC_AXIS_LEN};
     mw.y = {src + 3 * NOALLOC_AXIS_LEN, mul + 3 * NOALLOC_AXIS_LEN};
 
-    // tables into the scratch array; the solver's barrier state and status
-    // must start at zero (the planes are fully written before they are read)
+    // tables into the scratch array; the solver's status must start at zero (the
+    // planes are written before they are read, the exchange slots zeroed below)
     build_tables(*grid, NX, NY);
     if (cudaMemcpyAsync(metric, g_tab.metric, sizeof(g_tab.metric), cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaMemcpyAsync(mul, g_tab.mul, sizeof(g_tab.mul), cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -234,14 +238,18 @@ extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const 
     A.maxit = params->P_CG_MAXIT;
     A.partials = base + NA_OFF_PART;
     A.scal = scal;
-    const int n = (NX - 1) * (NY - 1);
-    const int nb = (n + NOALLOC_THREADS - 1) / NOALLOC_THREADS;   // one cell per thread: at most 141 blocks
-    if (nb > sc.coop_blocks) return na_err(PVOF_ECUDA, "the solver's blocks do not fit on the device at once");
+    // a cell per thread where the blocks are co-resident (at most 141, which every
+    // B200 holds; fewer SMs, as in an instance of a partitioned GPU, may not), else a
+    // walk of the range
+    const int n = (NX - 1) * (NY - 1), all = (n + NOALLOC_THREADS - 1) / NOALLOC_THREADS;
+    const bool resident = all <= std::min(sc.resident_blocks, most);
+    const int nb = resident ? all : std::max(1, std::min(all, std::min(sc.walk_blocks, most)));
+    const void *fn = resident ? (const void *)k_cg_pressure : (const void *)k_cg_pressure_walk;
     // the solver's exchange slots start from epoch zero
     if (cudaMemsetAsync(base + NA_OFF_PART, 0, SLOT_DOUBLES * (size_t)(nb + 1) * sizeof(double), st) != cudaSuccess)
         return na_err(PVOF_ECUDA, "scratch set-up failed");
     void *args[] = {&A};
-    if (cudaLaunchCooperativeKernel((const void *)k_cg_pressure, dim3((unsigned)nb), dim3(NOALLOC_THREADS), args, 0, st) !=
+    if (cudaLaunchCooperativeKernel(fn, dim3((unsigned)nb), dim3(NOALLOC_THREADS), args, 0, st) !=
         cudaSuccess)
         return na_err(PVOF_ECUDA, "solver launch failed");
 
@@ -258,4 +266,12 @@ extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const 
     if (iterations) *iterations = h.p_iters;
     if (residual) *residual = h.p_res;
     return h.p_iters;
+}
+
+// See the file comment and include/pvof.h.
+extern "C" int pvof_Pressure_solve_cg_noalloc(const pvof_grid_desc *grid, const pvof_params *params,
+                                              const double *rho, const double *rhs, double *phi, void *stream,
+                                              int *iterations, double *residual)
+{
+    return pvof_noalloc_solve(grid, params, rho, rhs, phi, stream, iterations, residual, NOALLOC_MAX_BLOCKS);
 }
