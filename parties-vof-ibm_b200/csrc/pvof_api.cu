@@ -1724,12 +1724,13 @@ int p_solve_fft(pvof_ctx *c)
     A.inx = 1.0 / (d.NX - 1.0);
     A.rx = fft_radices(N);
     A.ry = fft_radices(NYp);
-    // Rows and columns per block: up to 4 KB-sized transforms together, as
-    // long as every SM still has a block.  The y solve by cosine transforms
+    // Rows and columns per block: short transforms together up to 1024 and 4096
+    // points (16 and 64 KB a buffer), as long as every SM still has a block.  The y
+    // solve by cosine transforms
     // needs two buffers of a column in shared memory (7000 rows), and a prime
     // factor p costs p operations per value and pass: up to 31 the transforms
     // are ahead of the Thomas chain (1024x2048 1200 -> 51 us, 200x800 470 -> 11 us).
-    const int H = N / 2 + 1, sms = 148;
+    const int H = N / 2 + 1, sms = c->sms;
     A.pairs = std::max(1, std::min(std::min(8, 1024 / N), NYp / 2 / sms));
     A.cols = 0;
     if (A.ry.largest <= 31 && NYp <= 7000)
@@ -1953,6 +1954,7 @@ int pvof_create(const pvof_grid_desc *grid, const pvof_params *params, int devic
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     if (!coop) return fail(PVOF_ENODEV, "device without cooperative launch");
+    c->sms = nsm;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, k_cg_biharmonic, COOP_THREADS, 0);
     {
         int o1f = 0;

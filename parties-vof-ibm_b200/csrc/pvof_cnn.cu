@@ -741,6 +741,14 @@ int *cnn_error()
     return cudaGetSymbolAddress((void **)&err, g_cnn_err) == cudaSuccess ? err : nullptr;
 }
 
+// multiprocessors of the current device
+int device_sms()
+{
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+    return n;
+}
+
 // A hidden layer's convolution, forward (mask null) or input gradient through
 // the ReLU mask of the layer below.  Tiles of 8 rows where they fill the SMs,
 // else of 4 or 2 (more CTAs; a tile's halo rows are read again by its
@@ -760,9 +768,9 @@ template <bool DGRAD>
 int conv32(const float *in, const __nv_bfloat16 *w, const float *b, float *out, const float *mask, int H, int W, int relu,
            cudaStream_t st)
 {
-    const long long ns = um_strips(W);
-    if (ns * (H / 8) >= 148) return conv32_launch<8, DGRAD>(in, w, b, out, mask, H, W, relu, st);
-    if (ns * (H / 4) >= 148) return conv32_launch<4, DGRAD>(in, w, b, out, mask, H, W, relu, st);
+    const long long ns = um_strips(W), sms = device_sms();
+    if (ns * (H / 8) >= sms) return conv32_launch<8, DGRAD>(in, w, b, out, mask, H, W, relu, st);
+    if (ns * (H / 4) >= sms) return conv32_launch<4, DGRAD>(in, w, b, out, mask, H, W, relu, st);
     return conv32_launch<2, DGRAD>(in, w, b, out, mask, H, W, relu, st);
 }
 
@@ -922,7 +930,7 @@ int pvof_cnn_forward(const float *params, const uint16_t *params_bf16, const flo
     const Layer &Z = L[CNN_LAYERS - 1];   // the last: one plane, and y
     float *y0 = work + (size_t)(CNN_LAYERS - 1) * CNN_CMAX * plane;
     const unsigned gx = (unsigned)((W + 31) / 32), gy4 = (unsigned)((H + 31) / 32);
-    if (gx * gy4 >= 148) k_conv_last<4><<<dim3(gx, gy4), 256, 0, st>>>(in, wb + Z.w, params + Z.b, y0, y, H, W);
+    if (gx * gy4 >= (unsigned)device_sms()) k_conv_last<4><<<dim3(gx, gy4), 256, 0, st>>>(in, wb + Z.w, params + Z.b, y0, y, H, W);
     else k_conv_last<1><<<dim3(gx, (unsigned)((H + 7) / 8)), 256, 0, st>>>(in, wb + Z.w, params + Z.b, y0, y, H, W);
     return cudaGetLastError() == cudaSuccess ? PVOF_OK : PVOF_ECUDA;
 }

@@ -137,7 +137,7 @@ struct GraphEntry {
 struct Ctx {
     pvof_grid_desc g;
     pvof_params p;
-    int device;
+    int device, sms;         // its multiprocessors
     Dom dom;
     size_t plane_elems;      // P * (NY + 2*NG)
     double *base[PVOF_F_COUNT];   // allocation bases
