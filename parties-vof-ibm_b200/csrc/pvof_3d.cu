@@ -320,9 +320,13 @@ __global__ void __launch_bounds__(256) k3p_dir(Dom3 d, const double *__restrict_
 }
 
 // The momentum PCG's two passes over the faces of component C (one face per
-// thread in PKB planes), as above.  KC: the direction's ghost update.
-// 120x97x104, an iteration: 78 us in five launches (the weights already
-// stored) -> 63 us in two.
+// thread in PKB planes).  First pass: x += alpha d_old of the iteration before,
+// the direction d = z + beta d_old, A d and d.Ad; a thread marches its planes with
+// the directions of three planes in registers.  KC: the direction's ghost update.
+// Second pass: r -= alpha Ad, z = M^-1 r and the sums.  One face a thread leaves
+// room for four blocks per SM, where two pressure cells left three.  Bound by HBM
+// at 256^3, by latency and launches below.  120x97x104, an iteration: 78 us in
+// five launches (the weights already stored) -> 63 us in two.
 template <int C, int KC, class F>
 __global__ void __launch_bounds__(256, 4) k3v_dir_op(Dom3 d, Range r, double iRe, const double *__restrict__ FT,
                                                   const double *__restrict__ MU, const double *__restrict__ MA,

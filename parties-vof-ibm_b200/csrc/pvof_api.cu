@@ -1725,11 +1725,11 @@ int p_solve_fft(pvof_ctx *c)
     A.rx = fft_radices(N);
     A.ry = fft_radices(NYp);
     // Rows and columns per block: short transforms together up to 1024 and 4096
-    // points (16 and 64 KB a buffer), as long as every SM still has a block.  The y
-    // solve by cosine transforms
-    // needs two buffers of a column in shared memory (7000 rows), and a prime
-    // factor p costs p operations per value and pass: up to 31 the transforms
-    // are ahead of the Thomas chain (1024x2048 1200 -> 51 us, 200x800 470 -> 11 us).
+    // points (16 and 64 KB a buffer), as long as every SM still has a block.  The
+    // y solve by cosine transforms needs two buffers of a column in shared memory
+    // (7000 rows), and a prime factor p costs p operations per value and pass: up
+    // to 31 the transforms are ahead of the Thomas chain (1024x2048 1200 -> 51 us,
+    // 200x800 470 -> 11 us).
     const int H = N / 2 + 1, sms = c->sms;
     A.pairs = std::max(1, std::min(std::min(8, 1024 / N), NYp / 2 / sms));
     A.cols = 0;
@@ -1770,7 +1770,12 @@ int p_solve_fft(pvof_ctx *c)
         }
         const double idx = hm.idx_u[NG];
         for (int i = 0; i < H; i++) mw[i] = 2.0 * (1 - cos(2. * pi * i / N)) * (idx * idx);
-        if (A.cols) {   // as the tridiagonal rows hold it, rounded into their diagonal
+        if (A.cols) {
+            // as the tridiagonal rows hold it, rounded to the grain of their diagonal:
+            // the solve agrees with the reference's elimination of the rounded matrix.
+            // Unrounded, a low wave number's eigenvalue would be as much as ten times
+            // closer to the exact operator's (1024 cells in x: 5e-13 instead of 1e-12 to
+            // 5e-12 at k = 2).
             const int m = NYp / 2;
             const double ap = -idy_v(m) * idy_c(m - 1) - idy_v(m) * idy_c(m);
             for (int i = 0; i < H; i++) mw[i] = ap - (ap - mw[i]);

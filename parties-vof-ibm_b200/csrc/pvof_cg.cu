@@ -1,27 +1,26 @@
 // Persistent iterative solvers of the two-phase substep.
 //
 // Each solve is ONE cooperative launch that runs the reference's whole CG
-// loop on the device: the blocks step through the iterations together,
-// separated by a grid barrier, and every block reduces the per-block partial
-// sums of each inner product in the same fixed order, so all blocks take the
-// same convergence decisions.  Cells are assigned to threads by the same
+// loop on the device: the blocks step through the iterations together, and the
+// exchange of the inner products' sums (grid_exchange) is the barrier between
+// its phases.  The sums are added in a fixed tree, by every block or by the
+// first one for all, so all blocks hold the same totals and take the same
+// convergence decisions.  Cells are assigned to threads by the same
 // grid-stride mapping in every phase, so a thread reads back its own cells'
 // private values (diagonal, Ad) without a barrier.
 //
-// Two grid barriers per iteration (three in the biharmonic solve): the new
-// search direction d_k = z_k + beta d_{k-1} is not written in a phase of its
-// own; the matrix-vector phase writes it for its own cells into the second
+// Two exchanges per iteration (three in the biharmonic solve through a field):
+// the new search direction d_k = z_k + beta d_{k-1} is not written in a phase of
+// its own; the matrix-vector phase writes it for its own cells into the second
 // direction buffer and evaluates it on the fly at the stencil neighbours (from
 // z and d_{k-1}, with the reference's ghost update of d applied through the
 // same source maps).  The arithmetic per value is the reference's, so the
 // iterates are those of the reference's loop.
 //
-// The grid barriers are this file's own (not cooperative_groups::grid_group::
-// sync) so that their waits are bounded: if the other blocks never arrive
-// they record an error in DevScalars::error and every block leaves the
-// solver.  The barrier is the exchange of the inner products' sums itself
-// (grid_exchange).  Ranges of at most one cell per resident thread keep the
-// whole solve in registers.
+// The waits are bounded (cooperative_groups::grid_group::sync's are not): if the
+// other blocks never arrive, an error is recorded in DevScalars::error and every
+// block leaves the solver.  Ranges of at most one cell per resident thread keep
+// the whole momentum or pressure solve in registers.
 #include "pvof_device.cuh"
 #include "pvof_exchange.cuh"
 #include "pvof_kernels.cuh"

@@ -29,16 +29,18 @@
 //   * the inner products are exchanged by pushes too: every CTA stores its sum
 //     into every CTA's shared memory (st.async, completing on the receiver's
 //     mbarrier together with the boundary rows), waits for the 16 sums on its own
-//     mbarrier and adds them in rank order, so every CTA takes the same
+//     mbarrier and adds them in a fixed tree over the ranks (the same in every
+//     CTA and run, so runs repeat bit for bit), so every CTA takes the same
 //     convergence decisions; the iteration's scalar arithmetic (alpha, beta, the
 //     stopping test) runs once per CTA and is broadcast with the sums.
 // Two exchanges per iteration, each one trip between CTAs where a cluster
 // barrier and a read of the other CTAs' sums behind it take three.  Bound by
 // the latency of the two exchanges and of the cells' chains between them;
 // 128x512, B200, with branch-free cell loops: pressure iteration 5.5 -> 4.6 us,
-// u and v momentum iteration 9.1 -> 5.4 us (whose weights are kept inverted
-// too, no division left in it).  The per-cell arithmetic is otherwise the
-// reference's: the same operands in the same order.
+// u and v momentum iteration 9.1 -> 5.4 us.  The per-cell arithmetic is the
+// reference's, the same operands in the same order, but for the momentum
+// solve's preconditioner: its diagonal is kept inverted (no division left in the
+// iteration), so z = r (1 / d) rounds once more than r / d.
 #include <algorithm>
 #include <cooperative_groups.h>
 #include <cstdlib>

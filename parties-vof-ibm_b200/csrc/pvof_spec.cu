@@ -44,8 +44,8 @@
 // so the solve stops at the same residual size; the iterates differ, so the
 // result moves within that tolerance of the reference's.
 //
-// The whole solve is ONE cooperative launch: blocks of SPEC_PT threads, eight
-// 128-thread row groups in the row phases, eight warps of one tridiagonal
+// The whole solve is ONE cooperative launch: blocks of SPEC_PT threads, four
+// 256-thread row groups in the row phases, eight warps of one tridiagonal
 // system each per block in the solve phase, four grid-wide exchanges per
 // iteration (grid_exchange: after the matrix-vector product, the update with
 // its forward transforms, the tridiagonal solves, the inverse transforms), one
