@@ -166,20 +166,19 @@ using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// looked up once, by whichever host thread comes first; the others wait for it
+// (contexts advanced together make their maps at the same time)
 EncodeTiled encode_fn()
 {
-    static EncodeTiled fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const EncodeTiled fn = [] {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
             q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiled)p;
-        else
-            cudaGetLastError();
-    }
+            return (EncodeTiled)p;
+        cudaGetLastError();
+        return (EncodeTiled) nullptr;
+    }();
     return fn;
 }
 
