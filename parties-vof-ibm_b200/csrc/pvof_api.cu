@@ -556,10 +556,15 @@ int vof_diffuse_init(pvof_ctx *c)
 // blocks at 64 registers, cost more than the third exchange of the form through a
 // field.  B200, us a solve, on the fly | field: 32x64 28.5 | 28.9, 64x300 38.0 |
 // 44.4, 128x512 40.0 | 44.9, 256x256 67.3 | 78.5, 296x256 (75 776 cells, the last)
-// 91 | 100, 300x256 115 | 103, 512x512 (64 registers) 527 | 399.
+// 91 | 100, 300x256 115 | 103, 512x512 (64 registers) 527 | 399.  Contexts
+// advanced together share the SMs, where the smaller blocks of the form through a
+// field let more solves run at once (a step of six droplets 64 to 192 cells across:
+// 20.1 ms on the fly, 18.6 through the field).
+// Both give the same bits: the same operands and, up to a cell per thread, the
+// same sums.
 bool biharmonic_on_the_fly(const pvof_ctx *c)
 {
-    return (c->dom.NX - 1) * (c->dom.NY - 1) <= c->bih_fly_blocks * COOP_THREADS;
+    return !c->vel_one_cluster && (c->dom.NX - 1) * (c->dom.NY - 1) <= c->bih_fly_blocks * COOP_THREADS;
 }
 
 int vof_diffuse_step(pvof_ctx *c)

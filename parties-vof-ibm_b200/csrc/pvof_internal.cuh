@@ -161,7 +161,7 @@ struct Ctx {
     size_t cgs_v_smem;       // same, velocity solver for both components (0: grid solver)
     int cgs_p_threads, cgs_v_threads;   // their threads per CTA
     StripPlan cgs_p_fit, cgs_v_fit;     // the cluster plans that fit this grid (kept for pvof_set_cluster_solvers)
-    int vel_one_cluster;     // momentum solve as u then v on one cluster (batched runs)
+    int vel_one_cluster;     // advanced with other contexts: momentum solve as u then v on one cluster
     int pressure_pairs;      // grid-wide pressure solve over pairs of cells: -1 by size, 0 never, 1 always
     int phi_prev_mask;       // stages whose last correction is kept in SC_PHI_PREV + stage
     int phi_old_mask;        // stages whose correction one step before that is in SC_PHI_OLD + stage
